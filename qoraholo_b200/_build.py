@@ -31,7 +31,7 @@ BUILD = PKG / "_build"
 INCLUDE = ROOT / "include"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-std=c++20", "-O3", *ARCH, "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler",
+NVCC_FLAGS = ["-std=c++20", "-O3", "--split-compile=0", *ARCH, "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler",
               "-fPIC,-ffp-contract=off", f"-I{INCLUDE}", f"-I{CSRC}"]
 CXX_FLAGS = ["-std=c++20", "-O2", "-fPIC", "-ffp-contract=off", f"-I{INCLUDE}", f"-I{CSRC}"]
 

@@ -19,6 +19,7 @@
 #include <set>
 
 #include "autotune.hpp"
+#include "fft_two.hpp"
 #include "qhk_internal.hpp"
 
 namespace qhk {
@@ -739,6 +740,11 @@ void axis_pass(float2* data, int n_outer, std::size_t so, int n, std::size_t sp,
   if (engine != 0 && axis_pass_reg(data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb, engine)) {
     return;
   }
+  if (engine != 0 && axis_two_covers(n)) {
+    const int cols = tuned_choice(axis_key(n_outer, so, n, sp, ni, forward, mode, batch), axis_two_columns(n).front());
+    axis_pass_two(cols, data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb);
+    return;
+  }
   require(static_cast<std::size_t>(n) * 2 * sizeof(float2) <= 200 * 1024, "fft: transform length too large");
   const int cols = tuned_choice(axis_key(n_outer, so, n, sp, ni, forward, mode, batch), axis_default(n));
   axis_cols(cols, data, n_outer, so, n, sp, ni, forward, mode, scale, aux, batch, sb, s);
@@ -766,26 +772,26 @@ void tune_axis_pass(float2* data, int n_outer, std::size_t so, int n, std::size_
              s);
     return;
   }
+  if (axis_two_covers(n)) {
+    autotune(axis_key(n_outer, so, n, sp, ni, forward, mode, batch), axis_two_columns(n),
+             axis_two_columns(n).front(), [&](int c) {
+               axis_pass_two(c, data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb);
+             },
+             s);
+    return;
+  }
   autotune(axis_key(n_outer, so, n, sp, ni, forward, mode, batch), axis_candidates(n), axis_default(n),
            [&](int c) { axis_cols(c, data, n_outer, so, n, sp, ni, forward, mode, scale, aux, batch, sb, s); }, s);
 }
 
-// Lengths with compile-time row kernels (the common volume and image sides); others run the
-// runtime-length kernels.
-#define QHK_FIXED_LENGTHS(X) X(32) X(64) X(96) X(128) X(192) X(256) X(384) X(512)
+// The half length beyond the two engines above with compile-time row kernels; others run the run-time ones.
+constexpr int kFixedHalf = 512;
 
 void rows_r2c(const float* x, float2* e, std::size_t rows, int nx, bool clamp, cudaStream_t s) {
   require(nx >= 2 && nx % 2 == 0, "rfft: row length must be even");
   if (rows_r2c_reg(x, e, rows, nx, clamp, s)) return;
-  switch (nx / 2) {
-#define QHK_R2C(M)                                                \
-  case M:                                                         \
-    launch_r2c<rows_per_cta(M), M>(x, e, rows, nx, clamp, s);     \
-    return;
-    QHK_FIXED_LENGTHS(QHK_R2C)
-#undef QHK_R2C
-    default: break;
-  }
+  if (rows_r2c_two(x, e, rows, nx, clamp, s)) return;
+  if (nx == 2 * kFixedHalf) return launch_r2c<rows_per_cta(kFixedHalf), kFixedHalf>(x, e, rows, nx, clamp, s);
   switch (rows_per_cta(nx / 2)) {
     case 16: launch_r2c<16, 0>(x, e, rows, nx, clamp, s); break;
     case 8: launch_r2c<8, 0>(x, e, rows, nx, clamp, s); break;
@@ -799,15 +805,8 @@ void rows_c2r(const float2* e, float* x, std::size_t rows, int nx, C2rMode mode,
               cudaStream_t s) {
   require(nx >= 2 && nx % 2 == 0, "irfft: row length must be even");
   if (rows_c2r_reg(e, x, rows, nx, mode, nm2, inv_k02, s)) return;
-  switch (nx / 2) {
-#define QHK_C2R(M)                                                          \
-  case M:                                                                   \
-    launch_c2r<rows_per_cta(M), M>(e, x, rows, nx, mode, nm2, inv_k02, s);  \
-    return;
-    QHK_FIXED_LENGTHS(QHK_C2R)
-#undef QHK_C2R
-    default: break;
-  }
+  if (rows_c2r_two(e, x, rows, nx, mode, nm2, inv_k02, s)) return;
+  if (nx == 2 * kFixedHalf) return launch_c2r<rows_per_cta(kFixedHalf), kFixedHalf>(e, x, rows, nx, mode, nm2, inv_k02, s);
   switch (rows_per_cta(nx / 2)) {
     case 16: launch_c2r<16, 0>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
     case 8: launch_c2r<8, 0>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
@@ -820,15 +819,8 @@ void rows_c2r(const float2* e, float* x, std::size_t rows, int nx, C2rMode mode,
 void rows_c2r_r2c(float2* e, std::size_t rows, int nx, cudaStream_t s) {
   require(nx >= 2 && nx % 2 == 0, "rfft: row length must be even");
   if (rows_c2r_r2c_reg(e, rows, nx, s)) return;
-  switch (nx / 2) {
-#define QHK_C2R_R2C(M)                                    \
-  case M:                                                 \
-    launch_c2r_r2c<rows_per_cta(M), M>(e, rows, nx, s);   \
-    return;
-    QHK_FIXED_LENGTHS(QHK_C2R_R2C)
-#undef QHK_C2R_R2C
-    default: break;
-  }
+  if (rows_c2r_r2c_two(e, rows, nx, s)) return;
+  if (nx == 2 * kFixedHalf) return launch_c2r_r2c<rows_per_cta(kFixedHalf), kFixedHalf>(e, rows, nx, s);
   switch (rows_per_cta(nx / 2)) {
     case 16: launch_c2r_r2c<16, 0>(e, rows, nx, s); break;
     case 8: launch_c2r_r2c<8, 0>(e, rows, nx, s); break;
@@ -841,15 +833,8 @@ void rows_c2r_r2c(float2* e, std::size_t rows, int nx, cudaStream_t s) {
 void rows_tv_final_r2c(const float* b, const float* const p[3], int nz, int ny, int nx, float lambda, float momentum,
                        float* xprev, float2* e, cudaStream_t s) {
   require(nx >= 2 && nx % 2 == 0 && nz >= 1 && ny >= 1, "rfft: row length must be even");
-  switch (nx / 2) {
-#define QHK_TVF_R2C(M)                                                                           \
-  case M:                                                                                        \
-    launch_tv_final_r2c<rows_per_cta(M), M>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s);    \
-    return;
-    QHK_FIXED_LENGTHS(QHK_TVF_R2C)
-#undef QHK_TVF_R2C
-    default: break;
-  }
+  if (rows_tv_final_r2c_two(b, p, nz, ny, nx, lambda, momentum, xprev, e, s)) return;
+  if (nx == 2 * kFixedHalf) return launch_tv_final_r2c<rows_per_cta(kFixedHalf), kFixedHalf>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s);
   switch (rows_per_cta(nx / 2)) {
     case 16: launch_tv_final_r2c<16, 0>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
     case 8: launch_tv_final_r2c<8, 0>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
@@ -861,15 +846,7 @@ void rows_tv_final_r2c(const float* b, const float* const p[3], int nz, int ny, 
 
 void rows_c2c(float2* data, std::size_t rows, int nx, bool forward, RowMode mode, float scale, float* index,
               float nm2, float inv_k02, cudaStream_t s) {
-  switch (nx) {
-#define QHK_C2C(N)                                                                                        \
-  case N:                                                                                                 \
-    c2c_rows_dispatch<rows_per_cta(N), N>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s);  \
-    return;
-    QHK_FIXED_LENGTHS(QHK_C2C)
-#undef QHK_C2C
-    default: break;
-  }
+  if (rows_c2c_two(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s)) return;
   switch (rows_per_cta(nx)) {
     case 16: c2c_rows_dispatch<16, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
     case 8: c2c_rows_dispatch<8, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
@@ -878,8 +855,6 @@ void rows_c2c(float2* data, std::size_t rows, int nx, bool forward, RowMode mode
     default: c2c_rows_dispatch<1, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
   }
 }
-
-#undef QHK_FIXED_LENGTHS
 
 void fft2d(float2* data, int count, int n, bool forward, float scale, cudaStream_t s) {
   rows_c2c(data, static_cast<std::size_t>(count) * n, n, forward, RowMode::plain, 1.0f, nullptr, 0, 0, s);

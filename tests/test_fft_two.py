@@ -1,0 +1,41 @@
+"""Transforms on the two-factor lines and the passes built on them, at the lengths where their dispatch and
+their tiles change: every radix class (2^a 3^b 5^c up to 16, 25 and 32, and factors 7, 11, 13), equal and
+unequal factors, the smallest lines, lengths without two radices (the staged engine), and planes up to the
+largest that fits a CTA's shared memory.
+
+The transform bound is 1e-6 in the relative 2-norm: a float32 FFT of n points errs by about
+eps log2(n) / 2 = 6e-8 * 9 / 2 per axis; three axes at n = 512 give under 1e-6."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+G = np.array([0.532, 1.337, 1.2, 0.2], np.float32)
+LENGTHS = [4, 6, 10, 14, 22, 26, 34, 62, 66, 78, 90, 96, 126, 154, 160, 182, 200, 208, 250, 286, 300, 320, 336, 352,
+           384, 390, 400, 416, 448, 480, 512]
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+def test_transforms_of_every_length_class(cuda, n):
+    from qoraholo_b200 import capi
+
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n))).astype(np.complex64)
+    for forward, fft in ((True, np.fft.fft2), (False, lambda a: np.fft.ifft2(a) * n * n)):
+        d = cuda.from_numpy(x).cuda()
+        capi.fft2d(d.data_ptr(), 3, n, forward, 0.5)
+        assert rel_err(d.cpu().numpy(), 0.5 * fft(x.astype(np.complex128))) < 1e-6
+    nz, ny = 6, 9  # an odd number of rows: the last one is transformed alone
+    r = rng.standard_normal((nz - 1, ny, n)).astype(np.float32)
+    want = np.fft.rfftn(r.astype(np.float64))
+    d, h = cuda.from_numpy(r).cuda(), cuda.empty((nz - 1, ny, n // 2 + 1), dtype=cuda.complex64, device="cuda")
+    capi.rfft3(d.data_ptr(), h.data_ptr(), nz - 1, ny, n)
+    assert rel_err(h.cpu().numpy(), want) < 1e-6
+    back = cuda.empty_like(d)
+    h = cuda.from_numpy(want.astype(np.complex64)).cuda()
+    capi.irfft3(h.data_ptr(), back.data_ptr(), nz - 1, ny, n, 1.0 / r.size)
+    assert rel_err(back.cpu().numpy(), r) < 1e-6
