@@ -363,19 +363,19 @@ void OdtPlan::tune() {
     for (const bool fwd : {true, false}) {
       tune_axis_pass(scratch, b * nz, nh, n, h, h, fwd, AxisMode::plain, 1.0f, AxisAux{}, s);
     }
-    tune_axis_pass(scratch, n, h, nz, nh, h, false, AxisMode::from_data, 1.0f, aux, s, b, half_);
-    tune_axis_pass(scratch, n, h, nz, nh, h, true, AxisMode::restore_half, 1.0f, aux, s, b, half_);
+    tune_axis_pass(scratch, 1, nh, nz, nh, static_cast<int>(nh), false, AxisMode::from_data, 1.0f, aux, s, b, half_);
+    tune_axis_pass(scratch, 1, nh, nz, nh, static_cast<int>(nh), true, AxisMode::restore_half, 1.0f, aux, s, b, half_);
     if (cfg_.tv) tune_tv(x_.get(), tv_[0], nz, n, n, cfg_.lambda, s);
   } else {
     for (const bool fwd : {true, false}) {
       tune_axis_pass(scratch, b * nz, nn, n, static_cast<std::size_t>(n), n, fwd, AxisMode::plain, 1.0f, AxisAux{},
                      s);
-      tune_axis_pass(scratch, n, static_cast<std::size_t>(n), nz, nn, n, fwd, AxisMode::plain, 1.0f, AxisAux{}, s,
+      tune_axis_pass(scratch, 1, nn, nz, nn, static_cast<int>(nn), fwd, AxisMode::plain, 1.0f, AxisAux{}, s,
                      b, vol_);
     }
     if (cfg_.iterations > 0) {
       check(cudaMemsetAsync(mask_.get(), 0, mask_.bytes(), s), "cudaMemset");
-      tune_axis_pass(scratch, n, static_cast<std::size_t>(n), nz, nn, n, true, AxisMode::restore_mask, 1.0f,
+      tune_axis_pass(scratch, 1, nn, nz, nn, static_cast<int>(nn), true, AxisMode::restore_mask, 1.0f,
                      AxisAux{measured_.get(), mask_.get()}, s, b, vol_);
     }
   }
@@ -436,8 +436,10 @@ void OdtPlan::solve_real(float* index, float inv, cudaStream_t s) {
   const std::size_t rows = static_cast<std::size_t>(b) * nz * n;
   float2* e = e_.get();
   const AxisAux aux{a_.get(), hits_.get()};
-  // E = a * inv, inverse along z, then y, then C2R along x.
-  axis_pass(e, n, h, nz, nh, h, false, AxisMode::from_data, inv, aux, s, b, half_);
+  // E = a * inv, inverse along z, then y, then C2R along x. The z passes take a plane's n h columns as one run:
+  // tiles straddle its rows, so none is ragged and all start on a 128-byte boundary (256^3, 129 bins per row:
+  // 47 us for the pass with the restore, from 53).
+  axis_pass(e, 1, nh, nz, nh, static_cast<int>(nh), false, AxisMode::from_data, inv, aux, s, b, half_);
   axis_pass(e, b * nz, nh, n, h, h, false, AxisMode::plain, 1.0f, AxisAux{}, s);
   if (!cfg_.tv) {
     // GP: x = C2R(E); each step clamps x, R2C, y, z restore, y, C2R. The C2R, the clamp and the next
@@ -445,7 +447,7 @@ void OdtPlan::solve_real(float* index, float inv, cudaStream_t s) {
     for (int it = 0; it < cfg_.iterations; ++it) {
       rows_c2r_r2c(e, rows, n, s);
       axis_pass(e, b * nz, nh, n, h, h, true, AxisMode::plain, 1.0f, AxisAux{}, s);
-      axis_pass(e, n, h, nz, nh, h, true, AxisMode::restore_half, inv, aux, s, b, half_);
+      axis_pass(e, 1, nh, nz, nh, static_cast<int>(nh), true, AxisMode::restore_half, inv, aux, s, b, half_);
       axis_pass(e, b * nz, nh, n, h, h, false, AxisMode::plain, 1.0f, AxisAux{}, s);
     }
     rows_c2r(e, index, rows, n, C2rMode::index, cfg_.nm2, cfg_.inv_k02, s);
@@ -455,7 +457,7 @@ void OdtPlan::solve_real(float* index, float inv, cudaStream_t s) {
   const auto kspace_step = [&](const float* in, bool clamp, float* out, C2rMode mode) {
     rows_r2c(in, e, rows, n, clamp, s);
     axis_pass(e, b * nz, nh, n, h, h, true, AxisMode::plain, 1.0f, AxisAux{}, s);
-    axis_pass(e, n, h, nz, nh, h, true, AxisMode::restore_half, inv, aux, s, b, half_);
+    axis_pass(e, 1, nh, nz, nh, static_cast<int>(nh), true, AxisMode::restore_half, inv, aux, s, b, half_);
     axis_pass(e, b * nz, nh, n, h, h, false, AxisMode::plain, 1.0f, AxisAux{}, s);
     rows_c2r(e, out, rows, n, mode, cfg_.nm2, cfg_.inv_k02, s);
   };
@@ -478,7 +480,7 @@ void OdtPlan::solve_real(float* index, float inv, cudaStream_t s) {
     } else {
       const NvtxRange r("qhk:kspace");
       axis_pass(e, b * nz, nh, n, h, h, true, AxisMode::plain, 1.0f, AxisAux{}, s);
-      axis_pass(e, n, h, nz, nh, h, true, AxisMode::restore_half, inv, aux, s, b, half_);
+      axis_pass(e, 1, nh, nz, nh, static_cast<int>(nh), true, AxisMode::restore_half, inv, aux, s, b, half_);
       axis_pass(e, b * nz, nh, n, h, h, false, AxisMode::plain, 1.0f, AxisAux{}, s);
       rows_c2r(e, x_.get(), rows, n, C2rMode::store, cfg_.nm2, cfg_.inv_k02, s);
     }
@@ -547,12 +549,12 @@ void OdtPlan::solve_complex(float* index, float inv, cudaStream_t s) {
   const std::size_t rows = static_cast<std::size_t>(b) * nz * n;
   float2* p = pot_.get();
   const AxisAux aux{measured_.get(), mask_.get()};
-  axis_pass(p, n, n, nz, nn, n, false, AxisMode::plain, 1.0f, AxisAux{}, s, b, vol_);
+  axis_pass(p, 1, nn, nz, nn, static_cast<int>(nn), false, AxisMode::plain, 1.0f, AxisAux{}, s, b, vol_);
   axis_pass(p, b * nz, nn, n, n, n, false, AxisMode::plain, 1.0f, AxisAux{}, s);
   for (int it = 0; it < cfg_.iterations; ++it) {
     rows_c2c(p, rows, n, false, RowMode::inv_clamp_fwd, inv, nullptr, 0, 0, s);
     axis_pass(p, b * nz, nn, n, n, n, true, AxisMode::plain, 1.0f, AxisAux{}, s);
-    axis_pass(p, n, n, nz, nn, n, true, AxisMode::restore_mask, 1.0f, aux, s, b, vol_);
+    axis_pass(p, 1, nn, nz, nn, static_cast<int>(nn), true, AxisMode::restore_mask, 1.0f, aux, s, b, vol_);
     axis_pass(p, b * nz, nn, n, n, n, false, AxisMode::plain, 1.0f, AxisAux{}, s);
   }
   rows_c2c(p, rows, n, false, RowMode::inv_index, inv, index, cfg_.nm2, cfg_.inv_k02, s);
