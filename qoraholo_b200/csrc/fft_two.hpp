@@ -1,5 +1,5 @@
-// Host interface of the passes on the two-factor line transforms (fft_two.cu). Each returns
-// false when it does not cover the length, and has then done nothing.
+// Host interface of the passes on the two-factor line transforms (fft_two.cu, fft_plane.cu). Each returns
+// false when it does not cover the length (or the plane does not fit), and has then done nothing.
 #pragma once
 
 #include <vector>
@@ -24,5 +24,10 @@ bool rows_tv_final_r2c_two(const float* b, const float* const p[3], int nz, int 
                            float momentum, float* xprev, float2* e, cudaStream_t s);
 bool rows_c2c_two(float2* data, std::size_t rows, int nx, bool forward, RowMode mode, float scale, float* index,
                   float nm2, float inv_k02, cudaStream_t s);
+
+// One Gerchberg-Papoulis step between two z passes, in place on `planes` half-spectrum planes (n, n / 2 + 1):
+// inverse y transform, C2R, max(x, 0), R2C, forward y transform, a plane on chip throughout.
+bool plane_gp_covers(int n);
+bool plane_gp(float2* e, std::size_t planes, int n, cudaStream_t s);
 
 }  // namespace qhk

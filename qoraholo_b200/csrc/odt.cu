@@ -19,6 +19,7 @@
 
 #include "autotune.hpp"
 #include "debug.cuh"
+#include "fft_two.hpp"
 #include "odt.hpp"
 #include "nvtx.hpp"
 
@@ -440,6 +441,17 @@ void OdtPlan::solve_real(float* index, float inv, cudaStream_t s) {
   // tiles straddle its rows, so none is ragged and all start on a 128-byte boundary (256^3, 129 bins per row:
   // 47 us for the pass with the restore, from 53).
   axis_pass(e, 1, nh, nz, nh, static_cast<int>(nh), false, AxisMode::from_data, inv, aux, s, b, half_);
+  if (!cfg_.tv && cfg_.iterations > 0 && plane_gp_covers(n)) {
+    // GP with whole planes on chip: each step is a plane pass (inverse y, C2R, clamp, R2C, forward y) and a
+    // z pass with the restore.
+    for (int it = 0; it < cfg_.iterations; ++it) {
+      plane_gp(e, static_cast<std::size_t>(b) * nz, n, s);
+      axis_pass(e, 1, nh, nz, nh, static_cast<int>(nh), true, AxisMode::restore_half, inv, aux, s, b, half_);
+    }
+    axis_pass(e, b * nz, nh, n, h, h, false, AxisMode::plain, 1.0f, AxisAux{}, s);
+    rows_c2r(e, index, rows, n, C2rMode::index, cfg_.nm2, cfg_.inv_k02, s);
+    return;
+  }
   axis_pass(e, b * nz, nh, n, h, h, false, AxisMode::plain, 1.0f, AxisAux{}, s);
   if (!cfg_.tv) {
     // GP: x = C2R(E); each step clamps x, R2C, y, z restore, y, C2R. The C2R, the clamp and the next

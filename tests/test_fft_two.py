@@ -39,3 +39,24 @@ def test_transforms_of_every_length_class(cuda, n):
     h = cuda.from_numpy(want.astype(np.complex64)).cuda()
     capi.irfft3(h.data_ptr(), back.data_ptr(), nz - 1, ny, n, 1.0 / r.size)
     assert rel_err(back.cpu().numpy(), r) < 1e-6
+
+
+@pytest.mark.parametrize("n", [4, 10, 12, 30, 34, 48, 66, 90, 96, 126, 150, 154, 160, 176, 182, 196, 200, 208, 210, 220,
+                               224, 226, 230])
+def test_gp_planes_against_the_oracle(cuda, n):
+    """GP with whole planes on chip (up to 224: 226 and 230 have no two radices, and 230 would not fit), for
+    every class of x factors; batches of planes that fill the GPU and that do not."""
+    from oracle import qh_oracle as O
+    from qoraholo_b200 import capi
+
+    il = O.circular_scan(3, 0.9, G)
+    rng = np.random.default_rng(n)
+    fields = (rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n))).astype(np.complex64) * 0.05
+    want, _ = O.reconstruct(fields, il, G, nz=4, iterations=2)
+    plan = capi.OdtPlan(n, 3, il, G, nz=4, iterations=2)
+    d, out = cuda.from_numpy(fields).cuda(), cuda.empty(plan.shape, dtype=cuda.float32, device="cuda")
+    plan.run(d.data_ptr(), out.data_ptr())
+    cuda.cuda.synchronize()
+    plan.close()
+    # 1e-5 of the contrast: ten transforms of 1e-6 each, and two steps that do not amplify them.
+    assert rel_err(out.cpu().numpy() - G[1], want - G[1]) < 1e-5
