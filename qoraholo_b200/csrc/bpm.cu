@@ -3,7 +3,7 @@
 // and follows the CPU form (src/cpu/bpm.cpp:18-243) and the tables of src/bpm.cpp:10-60.
 //
 // A pass of the model processes a chunk of nb illuminations at once, all planes (nb, n, n). Each
-// slice is two 2D FFTs. For n = 64, 128, 256 (the register-resident engine) a slice is two passes, each
+// slice is two 2D FFTs. For the sides the two-factor line transforms cover a slice is two passes, each
 // keeping a line of every plane on chip across a transform, the pointwise step and the opposite transform:
 //   forward:  columns [FFT (completing FFT(w)), S = c (q W + (1 - q) S), IFFT] ->
 //             rows [IFFT (completing IFFT(S)), x 1/n^2, store envelope, times the screen e^{i phase x_k},
@@ -23,6 +23,8 @@
 
 #include "bpm.hpp"
 #include "fft_reg.cuh"
+#include "fft_two.cuh"
+#include "fft_two.hpp"
 #include "nvtx.hpp"
 
 namespace qhk {
@@ -134,12 +136,9 @@ __global__ void __launch_bounds__(kThreads) k_cols(ColArgs a, FftLen L) {
   }
 }
 
-// The same two passes on the register-resident engine (fft_reg.cuh) for n = 64, 128, 256: rows with
-// R = 256 / T rows per CTA, T threads per row; columns with COLS = 256 / T columns per CTA, T threads
-// per column, the epilogue of k_cols applied to the positions each thread holds.
-template <bool Fwd, int T, int V>
+template <int T, int V>
 __global__ void __launch_bounds__(kThreads)
-    k_rows_reg(const float2* __restrict__ src, float2* __restrict__ dst, std::size_t rows, const float2* tw) {
+    k_rows_reg(float2* __restrict__ data, std::size_t rows, const float2* tw) {
   using Tile = regfft::RowTile<T>;
   constexpr int N = T * V;
   extern __shared__ float2 sm[];
@@ -148,100 +147,15 @@ __global__ void __launch_bounds__(kThreads)
   const bool live = row < rows;
   float2 v[V];
 #pragma unroll
-  for (int j = 0; j < V; ++j) v[j] = live ? src[row * N + t + T * j] : make_float2(0.f, 0.f);
-  regfft::line_fft<T, V, Fwd>(v, t, sm + r, Tile::A, Tile::B, tw);  // every row read before any write
+  for (int j = 0; j < V; ++j) v[j] = live ? data[row * N + t + T * j] : make_float2(0.f, 0.f);
+  regfft::line_fft<T, V, true>(v, t, sm + r, Tile::A, Tile::B, tw);  // every row read before any write
   if (live) {
 #pragma unroll
-    for (int j = 0; j < V; ++j) dst[row * N + t + T * j] = v[j];
+    for (int j = 0; j < V; ++j) data[row * N + t + T * j] = v[j];
   }
 }
 
-template <bool Fwd, int Mode, int T, int V>
-__global__ void __launch_bounds__(kThreads) k_cols_reg(ColArgs a, const float2* tw) {
-  constexpr int N = T * V, COLS = kThreads / T;
-  extern __shared__ float2 sm[];
-  const int c = static_cast<int>(threadIdx.x) % COLS, t = static_cast<int>(threadIdx.x) / COLS;
-  const int col = static_cast<int>(blockIdx.x) * COLS + c;
-  const bool live = col < N;
-  const std::size_t base = static_cast<std::size_t>(blockIdx.y) * N * N + (live ? col : 0);
-  float2 v[V];
-#pragma unroll
-  for (int j = 0; j < V; ++j) v[j] = live ? a.data[base + static_cast<std::size_t>(t + T * j) * N] : make_float2(0.f, 0.f);
-  regfft::line_fft<T, V, Fwd>(v, t, sm + c, T * COLS, COLS, tw);
-  if (!live) return;
-#pragma unroll
-  for (int j = 0; j < V; ++j) {
-    const int pos = t + T * j;
-    const std::size_t g = base + static_cast<std::size_t>(pos) * N;
-    const float2 vv = v[j];
-    if constexpr (Mode == kScreen) {
-      const float2 w = cscale(vv, a.inv);
-      if (a.store) a.store[g] = w;
-      float sn, cs;
-      sincosf(a.phase * a.x[static_cast<std::size_t>(pos) * N + col], &sn, &cs);
-      a.data[g] = cmul(make_float2(cs, sn), w);
-    } else if constexpr (Mode == kPropagate) {
-      const float2 cc = a.coef[g];
-      const float q = a.q[g];
-      const float2 sv = a.s[g];
-      const float tre = q * vv.x + (1.0f - q) * sv.x;
-      const float tim = q * vv.y + (1.0f - q) * sv.y;
-      a.s[g] = make_float2(cc.x * tre - cc.y * tim, cc.x * tim + cc.y * tre);
-    } else if constexpr (Mode == kScale) {
-      a.data[g] = cscale(vv, a.inv);
-    } else {
-      float2 gi = a.s[g];
-      if (a.has_back) gi = cadd(gi, vv);
-      else gi = vv;
-      const float2 cc = a.coef[g];
-      const float q = a.q[g];
-      const float ure = cc.x * gi.x + cc.y * gi.y;
-      const float uim = cc.x * gi.y - cc.y * gi.x;
-      a.data[g] = make_float2(q * ure, q * uim);
-      a.s[g] = make_float2((1.0f - q) * ure, (1.0f - q) * uim);
-    }
-  }
-}
-
-template <int T, int V>
-void fft2_reg(const float2* src, float2* dst, bool forward, int nb, int mode, const ColArgs& args, cudaStream_t s) {
-  constexpr int N = T * V;
-  const float2* tw = fft_len(N).tw;
-  const std::size_t rows = static_cast<std::size_t>(nb) * N;
-  {
-    using Tile = regfft::RowTile<T>;
-    const std::size_t smem = static_cast<std::size_t>(V) * Tile::A * sizeof(float2);
-    const unsigned grid = static_cast<unsigned>((rows + Tile::R - 1) / Tile::R);
-    const auto launch = [&](auto kernel) {
-      ensure_smem(kernel);
-      kernel<<<grid, kThreads, smem, s>>>(src, dst, rows, tw);
-    };
-    if (forward) {
-      launch(k_rows_reg<true, T, V>);
-    } else {
-      launch(k_rows_reg<false, T, V>);
-    }
-    check_launch("bpm rows");
-  }
-  ColArgs a = args;
-  a.data = dst;
-  constexpr int COLS = kThreads / T;
-  const std::size_t smem = static_cast<std::size_t>(N) * COLS * sizeof(float2);
-  const dim3 grid((N + COLS - 1) / COLS, nb);
-  const auto launch = [&](auto kernel) {
-    ensure_smem(kernel);
-    kernel<<<grid, kThreads, smem, s>>>(a, tw);
-  };
-  switch (mode) {
-    case kScreen: launch(k_cols_reg<false, kScreen, T, V>); break;
-    case kPropagate: launch(k_cols_reg<true, kPropagate, T, V>); break;
-    case kScale: launch(k_cols_reg<false, kScale, T, V>); break;
-    default: launch(k_cols_reg<true, kSplit, T, V>); break;
-  }
-  check_launch("bpm cols");
-}
-
-// One slice of the forward sweep as two passes on the register engine, each keeping a line of every
+// One slice of the forward sweep as two passes, each keeping a line of every
 // plane on chip across a transform, the pointwise step and the opposite transform:
 //   column pass (kPropInv): the forward column transform of the row-transformed envelope completes its
 //     2D FFT W; S = c (q W + (1 - q) S) (as the kPropagate epilogue) is stored; the inverse column
@@ -252,6 +166,22 @@ void fft2_reg(const float2* src, float2* dst, bool forward, int nb, int mode, co
 //     kScaleOut ends the sweep: inverse rows and x 1/n^2 only.
 // The inverse 2D FFT thus runs columns first and the forward one rows first; the recomputed segments use
 // the same two passes, so their envelopes are bitwise the forward sweep's.
+// The previous slice's gradient, added by the column pass: grad += gscale phase (part[0] + part[1] + ...),
+// groups in order. The image rows are shared out over the views' CTAs, a few each, so that no CTA of the pass
+// is held up by them; `t` of the `step` threads of column col.
+__device__ __forceinline__ void add_slice_gradient(const ColArgs& a, int n, int col, bool live, int t, int step) {
+  if (!a.grad || !live) return;
+  const std::size_t plane = static_cast<std::size_t>(n) * n;
+  const int views = static_cast<int>(gridDim.y), v = static_cast<int>(blockIdx.y);
+  const int last = n * (v + 1) / views;
+  for (int pos = n * v / views + t; pos < last; pos += step) {
+    const std::size_t p = static_cast<std::size_t>(pos) * n + col;
+    float acc = a.part[p];
+    for (int g = 1; g < a.groups; ++g) acc += a.part[g * plane + p];
+    a.grad[p] += a.gscale * a.phase * acc;
+  }
+}
+
 enum SliceMode : int { kPropInv = 0, kInvOnly = 1, kScreenFwd = 2, kScaleOut = 3, kSplitInv = 4 };
 
 template <int Mode, int T, int V>
@@ -284,16 +214,7 @@ __global__ void __launch_bounds__(kThreads) k_slice_cols(ColArgs a, const float2
   } else if constexpr (Mode == kSplitInv) {
     // Adjoint: the forward column transform completes FFT(w); U = conj(c)(g + back) (as the kSplit
     // epilogue), g = (1 - q) U is stored, b = q U goes on to the inverse column transform.
-    if (a.grad && blockIdx.y == 0 && live) {  // the previous slice's per-group sums, in group order
-      constexpr std::size_t plane = static_cast<std::size_t>(N) * N;
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
-        const std::size_t p = static_cast<std::size_t>(t + T * j) * N + col;
-        float acc = a.part[p];
-        for (int g = 1; g < a.groups; ++g) acc += a.part[g * plane + p];
-        a.grad[p] += a.gscale * a.phase * acc;
-      }
-    }
+    add_slice_gradient(a, N, col, live, t, T);
 #pragma unroll
     for (int j = 0; j < V; ++j) v[j] = live ? a.data[base + static_cast<std::size_t>(t + T * j) * N] : make_float2(0.f, 0.f);
     regfft::line_fft<T, V, true>(v, t, sm + c, T * COLS, COLS, tw);
@@ -420,6 +341,241 @@ __global__ void __launch_bounds__(kThreads)
   for (int j = 0; j < V; ++j) data[row + t + T * j] = v[j];
 }
 
+// The same passes on the two-factor line transforms (fft_two.cuh): the opposite transform runs on the values a
+// thread already holds, with the factors exchanged, in the same shared-memory slots.
+using twofft::Factors;
+
+// Columns per CTA of the column pass, and views (rows of one image row) per CTA of the row passes: small
+// CTAs, several per SM, whose loads overlap each other's transforms.
+constexpr int kSliceCols = 8;
+constexpr int kSliceLog = 3;
+constexpr int kSliceViews = 16;
+
+// Threads per CTA at most (the largest second factor per line), and CTAs per SM to leave registers for.
+constexpr int slice_threads(int max, int lines) { return std::min(max, 32) * lines; }
+constexpr int slice_blocks(int max, int lines) {
+  return (max == twofft::kSmall ? 768 : 512) / slice_threads(max, lines);
+}
+
+template <int Mode, int Max>
+__global__ void __launch_bounds__(slice_threads(Max, kSliceCols), slice_blocks(Max, kSliceCols))
+    k_slice_cols_two(ColArgs a, Factors f, const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  const int n = f.n(), A = (f.r2 | 1) * kSliceCols;
+  const int c = static_cast<int>(threadIdx.x) % kSliceCols, j = static_cast<int>(threadIdx.x) / kSliceCols;
+  const int col = static_cast<int>(blockIdx.x) * kSliceCols + c;
+  const bool live = col < n;
+  const std::size_t plane = static_cast<std::size_t>(n) * n;
+  const std::size_t base = static_cast<std::size_t>(blockIdx.y) * plane + (live ? col : 0);
+  const bool second = j < f.r1;
+  if constexpr (Mode == kSplitInv) {
+    add_slice_gradient(a, n, col, live, j, f.r2);
+  }
+  if constexpr (Mode != kInvOnly) {
+    twofft::with_first<Max>(f.r1, [&]<int R>() {
+      float2 v[R];
+      const float2* p = a.data + base + j * n;
+#pragma unroll
+      for (int q = 0; q < R; ++q, p += f.r2 * n) v[q] = live ? *p : make_float2(0.f, 0.f);
+      twofft::first_pass<R, true>(v, j, tw, sm + j * kSliceCols + c, A);
+    });
+    __syncthreads();
+  }
+  if (second) {
+    twofft::with_radix<Max>(f.r2, [&]<int R>() {
+      float2 u[R];
+      float2* x = sm + j * A + c;
+      if constexpr (Mode != kInvOnly) twofft::second_pass<R, true>(u, x, kSliceCols);
+      std::size_t g = base + static_cast<std::size_t>(j) * n;
+#pragma unroll
+      for (int q = 0; q < R; ++q, g += f.r1 * n) {
+        if constexpr (Mode == kInvOnly) {
+          u[q] = live ? a.s[g] : make_float2(0.f, 0.f);
+          continue;
+        }
+        if (!live) continue;
+        const float2 vv = u[q];
+        const float2 cc = a.coef[g];
+        const float w = a.q[g];
+        if constexpr (Mode == kPropInv) {
+          const float2 sv = a.s[g];
+          const float tre = w * vv.x + (1.0f - w) * sv.x;
+          const float tim = w * vv.y + (1.0f - w) * sv.y;
+          u[q] = make_float2(cc.x * tre - cc.y * tim, cc.x * tim + cc.y * tre);
+          a.s[g] = u[q];
+        } else {
+          // Adjoint: U = conj(c)(g + back) (as the kSplit epilogue), g = (1 - q) U is stored, b = q U goes on.
+          const float2 gi = a.has_back ? cadd(a.s[g], vv) : vv;
+          const float ure = cc.x * gi.x + cc.y * gi.y;
+          const float uim = cc.x * gi.y - cc.y * gi.x;
+          u[q] = make_float2(w * ure, w * uim);
+          a.s[g] = make_float2((1.0f - w) * ure, (1.0f - w) * uim);
+        }
+      }
+      twofft::first_pass<R, false>(u, j, tw, x, kSliceCols);
+    });
+  }
+  __syncthreads();
+  if (!live) return;
+  twofft::with_first<Max>(f.r1, [&]<int R>() {
+    float2 v[R];
+    twofft::second_pass<R, false>(v, sm + j * kSliceCols + c, A);
+    float2* p = a.data + base + j * n;
+#pragma unroll
+    for (int q = 0; q < R; ++q, p += f.r2 * n) *p = v[q];
+  });
+}
+
+// A row pass runs image row y (blockIdx.x) of one group of kSliceViews illuminations (blockIdx.y), so that
+// the group shares the screen factors of row y (computed once, in shared memory). Slots of a line: B = 1,
+// A = r2 | 1, lines C apart.
+__host__ __device__ __forceinline__ int slice_line_pitch(const Factors& f) { return f.r1 * (f.r2 | 1) + 1; }
+
+struct SliceRow {
+  int line, j, line2, j2;
+  bool first, second;          // has a butterfly of the first / the second pass
+  std::size_t row, row2;       // first elements of their rows
+};
+__device__ __forceinline__ SliceRow slice_row(const Factors& f, int nb) {
+  SliceRow r;
+  const int t = static_cast<int>(threadIdx.x), n = f.n();
+  r.line = t / f.r2;
+  r.j = t - r.line * f.r2;
+  r.line2 = t / f.r1;
+  r.j2 = t - r.line2 * f.r1;
+  const int v0 = static_cast<int>(blockIdx.y) * kSliceViews, y = static_cast<int>(blockIdx.x);
+  r.first = r.line < kSliceViews && v0 + r.line < nb;
+  r.second = r.line2 < kSliceViews && v0 + r.line2 < nb;
+  r.row = (static_cast<std::size_t>(r.first ? v0 + r.line : 0) * n + y) * n;
+  r.row2 = (static_cast<std::size_t>(r.second ? v0 + r.line2 : 0) * n + y) * n;
+  return r;
+}
+
+// (cos, sin) of phase x for the n pixels of image row y.
+__device__ __forceinline__ void row_screen(float2* screen, const float* x_row, int n, float phase) {
+  for (int p = static_cast<int>(threadIdx.x); p < n; p += static_cast<int>(blockDim.x)) {
+    float sn, cs;
+    sincosf(phase * x_row[p], &sn, &cs);
+    screen[p] = make_float2(cs, sn);
+  }
+}
+
+template <int Mode, int Max>
+__global__ void __launch_bounds__(slice_threads(Max, kSliceViews), slice_blocks(Max, kSliceViews))
+    k_slice_rows_two(ColArgs a, int nb, Factors f, const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  const int n = f.n(), A = f.r2 | 1, C = slice_line_pitch(f);
+  float2* screen = sm + kSliceViews * C;
+  const SliceRow r = slice_row(f, nb);
+  if (Mode == kScreenFwd) row_screen(screen, a.x + static_cast<std::size_t>(blockIdx.x) * n, n, a.phase);
+  if (r.first) {
+    twofft::with_first<Max>(f.r1, [&]<int R>() {
+      float2 v[R];
+      const float2* p = a.data + r.row + r.j;
+#pragma unroll
+      for (int q = 0; q < R; ++q, p += f.r2) v[q] = *p;
+      twofft::first_pass<R, false>(v, r.j, tw, sm + r.line * C + r.j, A);
+    });
+  }
+  __syncthreads();  // also publishes `screen`
+  if (r.second) {
+    twofft::with_radix<Max>(f.r2, [&]<int R>() {
+      float2 u[R];
+      float2* x = sm + r.line2 * C + r.j2 * A;
+      twofft::second_pass<R, false>(u, x, 1);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int pos = r.j2 + f.r1 * q;
+        const float2 w = cscale(u[q], a.inv);
+        if constexpr (Mode == kScreenFwd) {
+          if (a.store) a.store[r.row2 + pos] = w;
+          u[q] = cmul(screen[pos], w);
+        } else {
+          a.data[r.row2 + pos] = w;
+        }
+      }
+      if constexpr (Mode == kScreenFwd) twofft::first_pass<R, true>(u, r.j2, tw, x, 1);
+    });
+  }
+  if constexpr (Mode == kScreenFwd) {
+    __syncthreads();
+    if (r.first) {
+      twofft::with_first<Max>(f.r1, [&]<int R>() {
+        float2 v[R];
+        twofft::second_pass<R, true>(v, sm + r.line * C + r.j, A);
+        float2* p = a.data + r.row + r.j;
+#pragma unroll
+        for (int q = 0; q < R; ++q, p += f.r2) *p = v[q];
+      });
+    }
+  }
+}
+
+// Adjoint row pass of slice k: the inverse row transform completes IFFT(b); x 1/n^2; each view's term of the
+// gradient, Im(conj(t w_k) b) with t = e^{i phase x_k}, goes to shared memory, and one thread per pixel adds
+// the group's terms in view order into part[group, y, :]; b <- conj(t) b, then (kForward) the forward row
+// transform of the next slice's FFT. The next column pass, or k_gradient_groups, adds the groups in order
+// into the gradient.
+template <bool kForward, int Max>
+__global__ void __launch_bounds__(slice_threads(Max, kSliceViews), slice_blocks(Max, kSliceViews))
+    k_slice_gradient_two(float2* __restrict__ data, const float2* __restrict__ env, const float* __restrict__ x,
+                     float phase, float inv, int nb, float* __restrict__ part, Factors f,
+                     const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  const int n = f.n(), A = f.r2 | 1, C = slice_line_pitch(f);
+  float2* screen = sm + kSliceViews * C;
+  float* terms = reinterpret_cast<float*>(screen + n);  // kSliceViews x n
+  const SliceRow r = slice_row(f, nb);
+  const int y = static_cast<int>(blockIdx.x);
+  row_screen(screen, x + static_cast<std::size_t>(y) * n, n, phase);
+  if (r.first) {
+    twofft::with_first<Max>(f.r1, [&]<int R>() {
+      float2 v[R];
+      const float2* p = data + r.row + r.j;
+#pragma unroll
+      for (int q = 0; q < R; ++q, p += f.r2) v[q] = *p;
+      twofft::first_pass<R, false>(v, r.j, tw, sm + r.line * C + r.j, A);
+    });
+  }
+  __syncthreads();  // also publishes `screen`
+  if (r.second) {
+    twofft::with_radix<Max>(f.r2, [&]<int R>() {
+      float2 u[R];
+      float2* s = sm + r.line2 * C + r.j2 * A;
+      twofft::second_pass<R, false>(u, s, 1);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int pos = r.j2 + f.r1 * q;
+        const float cs = screen[pos].x, sn = screen[pos].y;
+        const float2 bv = cscale(u[q], inv);
+        const float2 w = cmul(make_float2(cs, sn), env[r.row2 + pos]);
+        terms[r.line2 * n + pos] = w.x * bv.y - w.y * bv.x;
+        u[q] = cmul(make_float2(cs, -sn), bv);
+        if constexpr (!kForward) data[r.row2 + pos] = u[q];
+      }
+      if constexpr (kForward) twofft::first_pass<R, true>(u, r.j2, tw, s, 1);
+    });
+  }
+  __syncthreads();
+  const int views = min(kSliceViews, nb - static_cast<int>(blockIdx.y) * kSliceViews);
+  for (int p = static_cast<int>(threadIdx.x); p < n; p += static_cast<int>(blockDim.x)) {
+    float acc = 0.0f;
+    for (int i = 0; i < views; ++i) acc += terms[i * n + p];
+    part[(static_cast<std::size_t>(blockIdx.y) * n + y) * n + p] = acc;
+  }
+  if constexpr (kForward) {
+    if (r.first) {
+      twofft::with_first<Max>(f.r1, [&]<int R>() {
+        float2 v[R];
+        twofft::second_pass<R, true>(v, sm + r.line * C + r.j, A);
+        float2* p = data + r.row + r.j;
+#pragma unroll
+        for (int q = 0; q < R; ++q, p += f.r2) *p = v[q];
+      });
+    }
+  }
+}
+
 // grad += gscale phase (part[0] + part[1] + ...), the groups added in order, per pixel.
 __global__ void k_gradient_groups(const float* __restrict__ part, int groups, std::size_t plane, float gscale,
                                   float phase, float* __restrict__ grad) {
@@ -431,20 +587,8 @@ __global__ void k_gradient_groups(const float* __restrict__ part, int groups, st
   }
 }
 
-// Calls f.template operator()<T, V>() for the plane sides the slice passes cover; false otherwise.
-template <class F>
-bool with_slice_shape(int n, F&& f) {
-  if (!fft_reg_engine_enabled()) return false;
-  switch (n) {
-    case 64: f.template operator()<8, 8>(); return true;
-    case 128: f.template operator()<8, 16>(); return true;
-    case 256: f.template operator()<16, 16>(); return true;
-    default: return false;
-  }
-}
-
 template <int T, int V>
-void slice_cols(int mode, const ColArgs& a, int nb, cudaStream_t s) {
+void slice_cols_reg(int mode, const ColArgs& a, int nb, cudaStream_t s) {
   constexpr int N = T * V, COLS = kThreads / T;
   const std::size_t smem = static_cast<std::size_t>(N) * COLS * sizeof(float2);
   const dim3 grid((N + COLS - 1) / COLS, nb);
@@ -464,7 +608,7 @@ void slice_cols(int mode, const ColArgs& a, int nb, cudaStream_t s) {
 }
 
 template <int T, int V>
-void slice_rows(int mode, const ColArgs& a, int nb, cudaStream_t s) {
+void slice_rows_reg(int mode, const ColArgs& a, int nb, cudaStream_t s) {
   using Tile = regfft::RowTile<T>;
   constexpr int N = T * V;
   const std::size_t smem = static_cast<std::size_t>(V) * Tile::A * sizeof(float2) + static_cast<std::size_t>(N) * sizeof(float2);
@@ -483,8 +627,8 @@ void slice_rows(int mode, const ColArgs& a, int nb, cudaStream_t s) {
 }
 
 template <int T, int V>
-void slice_gradient(bool forward, float2* data, const float2* env, const float* x, float phase, float inv, int nb,
-                    float gscale, float* part, float* grad, cudaStream_t s) {
+void slice_gradient_reg(bool forward, float2* data, const float2* env, const float* x, float phase, float inv, int nb,
+                        float* part, cudaStream_t s) {
   using Tile = regfft::RowTile<T>;
   constexpr int N = T * V;
   const int groups = (nb + Tile::R - 1) / Tile::R;
@@ -502,25 +646,144 @@ void slice_gradient(bool forward, float2* data, const float2* env, const float* 
     launch(k_slice_gradient<false, T, V>);
   }
   check_launch("bpm slice gradient");
-  if (grad) {  // else the next column pass adds the groups (ColArgs::grad)
-    const std::size_t plane = static_cast<std::size_t>(N) * N;
-    k_gradient_groups<<<static_cast<unsigned>((plane + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        part, groups, plane, gscale, phase, grad);
-    check_launch("bpm gradient groups");
-  }
 }
 
 // Forward rows only (the envelope of the first slice entering the sweep).
 template <int T, int V>
-void rows_forward(float2* data, int nb, cudaStream_t s) {
+void rows_forward_reg(float2* data, int nb, cudaStream_t s) {
   using Tile = regfft::RowTile<T>;
   constexpr int N = T * V;
   const std::size_t rows = static_cast<std::size_t>(nb) * N;
   const std::size_t smem = static_cast<std::size_t>(V) * Tile::A * sizeof(float2);
   const unsigned grid = static_cast<unsigned>((rows + Tile::R - 1) / Tile::R);
-  ensure_smem(k_rows_reg<true, T, V>);
-  k_rows_reg<true, T, V><<<grid, kThreads, smem, s>>>(data, data, rows, fft_len(N).tw);
+  ensure_smem(k_rows_reg<T, V>);
+  k_rows_reg<T, V><<<grid, kThreads, smem, s>>>(data, rows, fft_len(N).tw);
   check_launch("bpm rows");
+}
+
+template <int Max>
+void slice_cols_two(const Factors& f, int mode, const ColArgs& a, int nb, cudaStream_t s) {
+  const std::size_t smem = static_cast<std::size_t>(f.r1) * (f.r2 | 1) * kSliceCols * sizeof(float2);
+  const dim3 grid((f.n() + kSliceCols - 1) / kSliceCols, nb);
+  const float2* tw = fft_len(f.n()).tw;
+  const auto launch = [&](auto kernel) {
+    ensure_smem(kernel);
+    kernel<<<grid, f.r2 * kSliceCols, smem, s>>>(a, f, tw);
+  };
+  if (mode == kPropInv) {
+    launch(k_slice_cols_two<kPropInv, Max>);
+  } else if (mode == kSplitInv) {
+    launch(k_slice_cols_two<kSplitInv, Max>);
+  } else {
+    launch(k_slice_cols_two<kInvOnly, Max>);
+  }
+  check_launch("bpm slice columns");
+}
+
+template <int Max>
+void slice_rows_two(const Factors& f, int mode, const ColArgs& a, int nb, cudaStream_t s) {
+  const std::size_t smem = (static_cast<std::size_t>(kSliceViews) * slice_line_pitch(f) + f.n()) * sizeof(float2);
+  const dim3 grid(f.n(), (nb + kSliceViews - 1) / kSliceViews);
+  const float2* tw = fft_len(f.n()).tw;
+  const auto launch = [&](auto kernel) {
+    ensure_smem(kernel);
+    kernel<<<grid, f.r2 * kSliceViews, smem, s>>>(a, nb, f, tw);
+  };
+  if (mode == kScreenFwd) {
+    launch(k_slice_rows_two<kScreenFwd, Max>);
+  } else {
+    launch(k_slice_rows_two<kScaleOut, Max>);
+  }
+  check_launch("bpm slice rows");
+}
+
+template <int Max>
+void slice_gradient_two(const Factors& f, bool forward, float2* data, const float2* env, const float* x, float phase,
+                    float inv, int nb, float* part, cudaStream_t s) {
+  const int groups = (nb + kSliceViews - 1) / kSliceViews;
+  const std::size_t smem = (static_cast<std::size_t>(kSliceViews) * slice_line_pitch(f) + f.n()) * sizeof(float2) +
+                           static_cast<std::size_t>(kSliceViews) * f.n() * sizeof(float);
+  const float2* tw = fft_len(f.n()).tw;
+  const dim3 grid(f.n(), groups);
+  const auto launch = [&](auto kernel) {
+    ensure_smem(kernel);
+    kernel<<<grid, f.r2 * kSliceViews, smem, s>>>(data, env, x, phase, inv, nb, part, f, tw);
+  };
+  if (forward) {
+    launch(k_slice_gradient_two<true, Max>);
+  } else {
+    launch(k_slice_gradient_two<false, Max>);
+  }
+  check_launch("bpm slice gradient");
+}
+
+// The sides the slice passes cover, and the dispatch: 64, 128 and 256, whose lines have a compile-time form on
+// the register engine (256^2, 49 views: row pass 17 us, adjoint column pass 37 us, gradient pass 26 us, against
+// 26, 55 and 35 on the two-factor engine), take that; the others the two-factor engine (160^2, 24 views, per
+// slice: 9.3 and 6.9 us forward where the four staged passes took 39; the whole gradient of 60 slices 3.9 ms
+// from 8.6). Sides below 48 keep the staged passes: a slice of so small a plane is a few microseconds of launch
+// latency either way.
+Factors slice_factors(int n) {
+  Factors f;
+  twofft::factors(n, &f);
+  return f;
+}
+bool slice_covers(int n) {
+  Factors f;
+  return fft_reg_engine_enabled() && n >= 48 && twofft::factors(n, &f);
+}
+
+// Calls reg.template operator()<T, V>() or two.template operator()<Max>(factors).
+template <class Reg, class Two>
+void with_slice_shape(int n, Reg&& reg, Two&& two) {
+  switch (n) {
+    case 64: reg.template operator()<8, 8>(); return;
+    case 128: reg.template operator()<8, 16>(); return;
+    case 256: reg.template operator()<16, 16>(); return;
+    default: break;
+  }
+  const Factors f = slice_factors(n);
+  twofft::with_class(f, [&]<int Max>() { two.template operator()<Max>(f); });
+}
+
+// Views per group of the row passes (the groups the gradient is summed in).
+int slice_views(int n) { return n == 64 || n == 128 ? regfft::RowTile<8>::R : n == 256 ? regfft::RowTile<16>::R : kSliceViews; }
+
+void slice_cols(int n, int mode, const ColArgs& a, int nb, cudaStream_t s) {
+  with_slice_shape(
+      n, [&]<int T, int V>() { slice_cols_reg<T, V>(mode, a, nb, s); },
+      [&]<int Max>(const Factors& f) { slice_cols_two<Max>(f, mode, a, nb, s); });
+}
+
+void slice_rows(int n, int mode, const ColArgs& a, int nb, cudaStream_t s) {
+  with_slice_shape(
+      n, [&]<int T, int V>() { slice_rows_reg<T, V>(mode, a, nb, s); },
+      [&]<int Max>(const Factors& f) { slice_rows_two<Max>(f, mode, a, nb, s); });
+}
+
+// `grad`: add the groups now; otherwise the next column pass does (ColArgs::grad).
+void slice_gradient(int n, bool forward, float2* data, const float2* env, const float* x, float phase, float inv,
+                    int nb, float gscale, float* part, float* grad, cudaStream_t s) {
+  with_slice_shape(
+      n, [&]<int T, int V>() { slice_gradient_reg<T, V>(forward, data, env, x, phase, inv, nb, part, s); },
+      [&]<int Max>(const Factors& f) {
+        slice_gradient_two<Max>(f, forward, data, env, x, phase, inv, nb, part, s);
+      });
+  if (grad) {
+    const std::size_t plane = static_cast<std::size_t>(n) * n;
+    k_gradient_groups<<<static_cast<unsigned>((plane + kThreads - 1) / kThreads), kThreads, 0, s>>>(
+        part, (nb + slice_views(n) - 1) / slice_views(n), plane, gscale, phase, grad);
+    check_launch("bpm gradient groups");
+  }
+}
+
+// Forward rows only (the envelope of the first slice entering the sweep).
+void rows_forward(float2* data, int n, int nb, cudaStream_t s) {
+  with_slice_shape(
+      n, [&]<int T, int V>() { rows_forward_reg<T, V>(data, nb, s); },
+      [&]<int Max>(const Factors&) {
+        rows_c2c_two(data, static_cast<std::size_t>(nb) * n, n, true, RowMode::plain, 1.0f, nullptr, 0, 0, s);
+      });
 }
 
 // Spectrum of the unit envelope: n^2 at the zero bin of every plane.
@@ -734,17 +997,6 @@ std::size_t BpmPlan::device_bytes() const {
 void BpmPlan::fft2(const float2* src, float2* dst, bool forward, int nb, int mode, const void* args_v,
                    cudaStream_t s) {
   const int n = t_.n;
-  if (fft_reg_engine_enabled() && (n == 64 || n == 128 || n == 256)) {
-    const ColArgs& args = *static_cast<const ColArgs*>(args_v);
-    if (n == 64) {
-      fft2_reg<8, 8>(src, dst, forward, nb, mode, args, s);
-    } else if (n == 128) {
-      fft2_reg<8, 16>(src, dst, forward, nb, mode, args, s);
-    } else {
-      fft2_reg<16, 16>(src, dst, forward, nb, mode, args, s);
-    }
-    return;
-  }
   const FftLen& L = fft_len(n);
   const int c = rows_cols(n);
   const std::size_t rows = static_cast<std::size_t>(nb) * n;
@@ -806,34 +1058,33 @@ void BpmPlan::forward(const float* x, int first, int nb, cudaStream_t s) {
   k_first_screen<<<grid_for(total), kThreads, 0, s>>>(w_.get(), store_on_ ? stored_.get() : nullptr, x, t_.phase,
                                                       plane_, total);
   check_launch("bpm start");
-  // Two passes per slice on the register engine (k_slice_cols / k_slice_rows).
-  if (with_slice_shape(t_.n, [&]<int T, int V>() {
-        rows_forward<T, V>(w_.get(), nb, s);
-        for (int k = 0; k < nz; ++k) {
-          if (every_ > 0 && k % every_ == 0) {
-            float2* ck = ckpt_.get() + (static_cast<std::size_t>(k / every_) * t_.count + first) * plane_;
-            check(cudaMemcpyAsync(ck, s_.get(), total * sizeof(float2), cudaMemcpyDeviceToDevice, s),
-                  "bpm checkpoint");
-          }
-          ColArgs c{};
-          c.data = w_.get();
-          c.s = s_.get();
-          c.coef = (k == nz - 1 ? last_.get() : step_.get()) + off;
-          c.q = q_.get() + off;
-          slice_cols<T, V>(kPropInv, c, nb, s);
-          ColArgs w{};
-          w.data = w_.get();
-          w.inv = inv;
-          if (k + 1 < nz) {
-            w.store = store_on_ ? stored_.get() + (k + 1) * total : nullptr;
-            w.x = x + (k + 1) * plane_;
-            w.phase = t_.phase;
-            slice_rows<T, V>(kScreenFwd, w, nb, s);
-          } else {
-            slice_rows<T, V>(kScaleOut, w, nb, s);  // envelopes at z = 0 in w
-          }
-        }
-      })) {
+  // Two passes per slice on the two-factor engine (k_slice_cols / k_slice_rows).
+  if (slice_covers(t_.n)) {
+    rows_forward(w_.get(), t_.n, nb, s);
+    for (int k = 0; k < nz; ++k) {
+      if (every_ > 0 && k % every_ == 0) {
+        float2* ck = ckpt_.get() + (static_cast<std::size_t>(k / every_) * t_.count + first) * plane_;
+        check(cudaMemcpyAsync(ck, s_.get(), total * sizeof(float2), cudaMemcpyDeviceToDevice, s),
+              "bpm checkpoint");
+      }
+      ColArgs c{};
+      c.data = w_.get();
+      c.s = s_.get();
+      c.coef = (k == nz - 1 ? last_.get() : step_.get()) + off;
+      c.q = q_.get() + off;
+      slice_cols(t_.n, kPropInv, c, nb, s);
+      ColArgs w{};
+      w.data = w_.get();
+      w.inv = inv;
+      if (k + 1 < nz) {
+        w.store = store_on_ ? stored_.get() + (k + 1) * total : nullptr;
+        w.x = x + (k + 1) * plane_;
+        w.phase = t_.phase;
+        slice_rows(t_.n, kScreenFwd, w, nb, s);
+      } else {
+        slice_rows(t_.n, kScaleOut, w, nb, s);  // envelopes at z = 0 in w
+      }
+    }
     return;
   }
   for (int k = 0; k < nz; ++k) {
@@ -882,34 +1133,33 @@ void BpmPlan::adjoint(const float* x, const float2* residual_or_null, int first,
     }
     return stored_.get() + k * total;
   };
-  // Two passes per slice on the register engine: k_slice_gradient (inverse rows, gradient, conj(screen),
+  // Two passes per slice on the two-factor engine: k_slice_gradient (inverse rows, gradient, conj(screen),
   // forward rows) and k_slice_cols<kSplitInv> (forward columns, split, inverse columns).
-  if (with_slice_shape(t_.n, [&]<int T, int V>() {
-        const int groups = (nb + regfft::RowTile<T>::R - 1) / regfft::RowTile<T>::R;
-        const auto split = [&](const float2* coef, int has_back, float* slice_grad) {
-          ColArgs c{};
-          c.data = w_.get();
-          c.s = s_.get();
-          c.coef = coef + off;
-          c.q = q_.get() + off;
-          c.has_back = has_back;
-          c.part = gpart_.get();
-          c.groups = groups;
-          c.gscale = gscale;
-          c.phase = t_.phase;
-          c.grad = slice_grad;
-          slice_cols<T, V>(kSplitInv, c, nb, s);
-        };
-        rows_forward<T, V>(w_.get(), nb, s);
-        split(last_.get(), 0, nullptr);
-        for (int k = nz - 1; k >= 0; --k) {
-          const float2* env = envelope(k);
-          // Slice k's gradient groups are added by the next column pass, or here for the last slice.
-          slice_gradient<T, V>(k > 0, w_.get(), env, x + k * plane_, t_.phase, inv, nb, gscale, gpart_.get(),
-                               k > 0 ? nullptr : grad, s);
-          if (k > 0) split(step_.get(), 1, grad + k * plane_);
-        }
-      })) {
+  if (slice_covers(t_.n)) {
+    const int groups = (nb + slice_views(t_.n) - 1) / slice_views(t_.n);
+    const auto split = [&](const float2* coef, int has_back, float* slice_grad) {
+      ColArgs c{};
+      c.data = w_.get();
+      c.s = s_.get();
+      c.coef = coef + off;
+      c.q = q_.get() + off;
+      c.has_back = has_back;
+      c.part = gpart_.get();
+      c.groups = groups;
+      c.gscale = gscale;
+      c.phase = t_.phase;
+      c.grad = slice_grad;
+      slice_cols(t_.n, kSplitInv, c, nb, s);
+    };
+    rows_forward(w_.get(), t_.n, nb, s);
+    split(last_.get(), 0, nullptr);
+    for (int k = nz - 1; k >= 0; --k) {
+      const float2* env = envelope(k);
+      // Slice k's gradient groups are added by the next column pass, or here for the last slice.
+      slice_gradient(t_.n, k > 0, w_.get(), env, x + k * plane_, t_.phase, inv, nb, gscale, gpart_.get(),
+                           k > 0 ? nullptr : grad, s);
+      if (k > 0) split(step_.get(), 1, grad + k * plane_);
+    }
     return;
   }
   ColArgs a{};
@@ -943,38 +1193,37 @@ void BpmPlan::recompute(const float* x, int first, int nb, int k0, int k1, cudaS
   const float inv = 1.0f / static_cast<float>(plane_);
   const float2* ck = ckpt_.get() + (static_cast<std::size_t>(k0 / every_) * t_.count + first) * plane_;
   check(cudaMemcpyAsync(rs_.get(), ck, total * sizeof(float2), cudaMemcpyDeviceToDevice, s), "bpm restore");
-  // The forward sweep's two passes per slice (register engine), so the envelopes are bitwise its own.
-  if (with_slice_shape(t_.n, [&]<int T, int V>() {
-        const auto screen = [&](int k) {  // rw_ holds C^-1(S) of slice k: envelope k, then its row FFT
-          ColArgs w{};
-          w.data = rw_.get();
-          w.inv = inv;
-          w.store = env_.get() + (k - k0) * total;
-          w.x = x + k * plane_;
-          w.phase = t_.phase;
-          slice_rows<T, V>(kScreenFwd, w, nb, s);
-        };
-        if (k0 == 0) {
-          k_first_screen<<<grid_for(total), kThreads, 0, s>>>(rw_.get(), env_.get(), x, t_.phase, plane_, total);
-          check_launch("bpm recompute");
-          rows_forward<T, V>(rw_.get(), nb, s);
-        } else {
-          ColArgs c{};
-          c.data = rw_.get();
-          c.s = rs_.get();
-          slice_cols<T, V>(kInvOnly, c, nb, s);
-          screen(k0);
-        }
-        for (int k = k0; k + 1 < k1; ++k) {  // the spectrum entering k + 1, then envelope k + 1
-          ColArgs c{};
-          c.data = rw_.get();
-          c.s = rs_.get();
-          c.coef = step_.get() + off;
-          c.q = q_.get() + off;
-          slice_cols<T, V>(kPropInv, c, nb, s);
-          screen(k + 1);
-        }
-      })) {
+  // The forward sweep's two passes per slice (two-factor engine), so the envelopes are bitwise its own.
+  if (slice_covers(t_.n)) {
+    const auto screen = [&](int k) {  // rw_ holds C^-1(S) of slice k: envelope k, then its row FFT
+      ColArgs w{};
+      w.data = rw_.get();
+      w.inv = inv;
+      w.store = env_.get() + (k - k0) * total;
+      w.x = x + k * plane_;
+      w.phase = t_.phase;
+      slice_rows(t_.n, kScreenFwd, w, nb, s);
+    };
+    if (k0 == 0) {
+      k_first_screen<<<grid_for(total), kThreads, 0, s>>>(rw_.get(), env_.get(), x, t_.phase, plane_, total);
+      check_launch("bpm recompute");
+      rows_forward(rw_.get(), t_.n, nb, s);
+    } else {
+      ColArgs c{};
+      c.data = rw_.get();
+      c.s = rs_.get();
+      slice_cols(t_.n, kInvOnly, c, nb, s);
+      screen(k0);
+    }
+    for (int k = k0; k + 1 < k1; ++k) {  // the spectrum entering k + 1, then envelope k + 1
+      ColArgs c{};
+      c.data = rw_.get();
+      c.s = rs_.get();
+      c.coef = step_.get() + off;
+      c.q = q_.get() + off;
+      slice_cols(t_.n, kPropInv, c, nb, s);
+      screen(k + 1);
+    }
     return;
   }
   for (int k = k0; k < k1; ++k) {

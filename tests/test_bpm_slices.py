@@ -1,0 +1,38 @@
+"""The BPM slice passes at the sides where their dispatch changes (staged below 48 and without two radices,
+the register engine at 64, 128 and 256, the two-factor lines elsewhere, in each radix class) and with view
+counts around a group of the row passes, against the oracle."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+G = np.array([0.532, 1.337, 1.2, 0.2], np.float32)
+
+
+@pytest.mark.parametrize("n,count", [(46, 3), (48, 1), (62, 3), (64, 33), (66, 17), (78, 3), (100, 16), (154, 2),
+                                     (160, 17), (200, 2), (240, 3)])
+def test_slice_passes_match_the_oracle(cuda, n, count):
+    from oracle import qh_oracle as O
+    from qoraholo_b200.autograd import BpmModel
+
+    rng = np.random.default_rng(n)
+    nz = 5
+    il = O.circular_scan(count, 0.9, G)
+    ri = (G[1] + 0.03 * rng.random((nz, n, n))).astype(np.float32)
+    r = (rng.standard_normal((count, n, n)) + 1j * rng.standard_normal((count, n, n))).astype(np.complex64) * 0.1
+    want = O.bpm_forward(ri, il, G)
+    want_grad = O.bpm_vjp((ri - G[1]).astype(np.float32), r, O.bpm_tables(n, nz, il, G))
+    grads = []
+    for every in (2, 5):  # bitwise the same gradient whatever is stored
+        x = cuda.from_numpy(ri).cuda().requires_grad_(True)
+        y = BpmModel(nz, n, il, G, checkpoint_every=every)(x)
+        y.backward(cuda.from_numpy(r).cuda())
+        grads.append(x.grad.cpu().numpy())
+    # 2 transforms per slice of 1e-6 at most, forward; as many again back.
+    assert rel_err(y.detach().cpu().numpy(), want) < 1e-5
+    assert rel_err(grads[0], want_grad) < 2e-5
+    assert np.array_equal(grads[0], grads[1])
