@@ -20,6 +20,7 @@
 
 #include "debug.cuh"
 #include "fft_reg.cuh"
+#include "fft_two.cuh"
 #include "nvtx.hpp"
 #include "unwrap.hpp"
 
@@ -588,14 +589,387 @@ int unwrap_line_threads(int n) {
   return t;
 }
 
+// ---- The same three passes on two-factor lines (fft_two.cuh), for the other side lengths. The DCT runs through
+// the half-length transform as on the register engine above (the formulas of dct_pair and idct_merge), with
+// the factors at run time: h = n / 2 = r1 r2. Where h has no two radices because of a prime factor of 17 or
+// more (which the staged engine takes as a direct DFT per output, 4 p^2 multiplications for p of them, reading
+// every root from global memory), the second factor is any length: its DFT is a direct sum over pairs of
+// inputs (q, r2 - q) for pairs of outputs (m, r2 - m), r2^2 multiplications, four output pairs per thread
+// against shared roots. A tile has `lines` lines, the fastest index of every shared array, so that no
+// access has bank conflicts and no index needs a division. What bounds the passes is the latency of their
+// phases; 200 images of sides 96 .. 640 in steps of 8 (18 M pixels): the three passes take 0.96 ms, on the
+// staged engine 9.5 ms; one image of 120 x 160: 24 us from 40.
+struct DctLine {
+  int n = 0;  // side; 0: not on this engine
+  int r1 = 0, r2 = 0;
+  int direct = 0;  // the second factor is a direct sum
+  int lines = 0;   // lines per tile
+  __host__ __device__ int log_lines() const { return lines == 16 ? 4 : 3; }
+  __host__ __device__ int h() const { return n / 2; }
+  // float2 values of an exchange buffer (also h + 1 bins per line), and floats per staged row (odd: rows are
+  // read across lines).
+  __host__ __device__ int area() const { return (r1 * (r2 | 1) + 1) * lines; }
+  __host__ __device__ int pitch() const { return n + 1; }
+  __host__ __device__ std::size_t roots() const { return direct ? r2 : 0; }
+  __host__ __device__ std::size_t rows_smem() const {
+    return (2 * static_cast<std::size_t>(area()) + roots()) * sizeof(float2) +
+           static_cast<std::size_t>(lines + 2) * pitch() * sizeof(float);
+  }
+  __host__ __device__ std::size_t cols_smem() const {
+    return (2 * static_cast<std::size_t>(area()) + roots()) * sizeof(float2);
+  }
+};
+
+// The engine's line of length n; n = 0 in the result where the register or the staged engine runs it.
+DctLine dct_line(int n) {
+  DctLine l;
+  const int h = n / 2;
+  twofft::Factors f;
+  if (!fft_reg_engine_enabled() || n % 2 != 0 || h < 4) return l;
+  if (twofft::factors(h, &f)) {
+    l.r1 = f.r1;
+    l.r2 = f.r2;
+  } else {
+    int m = h, largest = 1;
+    for (int p = 2; m > 1; ++p) {
+      while (m % p == 0) m /= p, largest = p;
+    }
+    if (largest < 17 || h > 512) return l;
+    l.r1 = 16;
+    while (h % l.r1 != 0) --l.r1;
+    l.r2 = h / l.r1;
+    l.direct = 1;
+  }
+  l.n = n;
+  l.lines = n < 128 ? 16 : 8;
+  return l;
+}
+
+// First pass of the tile: load(line, m) gives input m of a line; slots (k1, j) of xs.
+template <bool Fwd, class Load>
+__device__ __forceinline__ void dct_first(const DctLine& f, float2* xs, const float2* __restrict__ twn, Load load) {
+  const int P = f.r2 | 1;
+  const auto run = [&]<int R>() {
+    for (int i = static_cast<int>(threadIdx.x); i < (f.r2 << f.log_lines()); i += kThreads) {
+      const int line = i & (f.lines - 1), j = i >> f.log_lines();
+      float2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = load(line, j + f.r2 * q);
+      twofft::dft<R, Fwd>(v);
+      float2* x = xs + (j << f.log_lines()) + line;
+      x[0] = v[0];
+#pragma unroll
+      for (int k1 = 1; k1 < R; ++k1) {
+        const float2 w = __ldg(twn + 2 * j * k1);
+        x[(k1 * P) << f.log_lines()] = Fwd ? cmul(v[k1], w) : cmulc(v[k1], w);
+      }
+    }
+  };
+  if (f.r1 == 1) {
+    run.template operator()<1>();
+  } else {
+    twofft::with_first<twofft::kAny>(f.r1, run);
+  }
+}
+
+// Second pass: sink(line, k, value) receives output k of a line.
+template <bool Fwd, class Sink>
+__device__ __forceinline__ void dct_second(const DctLine& f, const float2* xs, const float2* roots, Sink sink) {
+  const int P = f.r2 | 1, log = f.log_lines();
+  if (!f.direct) {
+    twofft::with_radix<twofft::kAny>(f.r2, [&]<int R>() {
+      for (int i = static_cast<int>(threadIdx.x); i < (f.r1 << log); i += kThreads) {
+        const int line = i & (f.lines - 1), k1 = i >> log;
+        float2 u[R];
+        twofft::second_pass<R, Fwd>(u, xs + ((k1 * P) << log) + line, f.lines);
+#pragma unroll
+        for (int q = 0; q < R; ++q) sink(line, k1 + f.r1 * q, u[q]);
+      }
+    });
+    return;
+  }
+  constexpr int MB = 4;
+  const int c = f.r2, pairs = (c - 1) / 2, outs = c / 2 + 1, blocks = (outs + MB - 1) / MB;
+  for (int i = static_cast<int>(threadIdx.x); i < ((f.r1 * blocks) << log); i += kThreads) {
+    const int line = i & (f.lines - 1), g = i >> log;
+    const int mb = g / f.r1, k1 = g - mb * f.r1, m0 = mb * MB;
+    const float2* x = xs + ((k1 * P) << log) + line;
+    float2 e[MB], d[MB];
+    int t[MB];
+    const float2 x0 = x[0];
+#pragma unroll
+    for (int b = 0; b < MB; ++b) {
+      e[b] = x0;
+      d[b] = make_float2(0.0f, 0.0f);
+      t[b] = 0;
+    }
+    for (int q = 1; q <= pairs; ++q) {
+      const float2 lo = x[q << log], hi = x[(c - q) << log];
+      const float2 a = cadd(lo, hi), s = csub(lo, hi);
+#pragma unroll
+      for (int b = 0; b < MB; ++b) {
+        t[b] += m0 + b;  // q m modulo c; m <= c / 2 + 3 < 2 c
+        while (t[b] >= c) t[b] -= c;
+        const float2 w = roots[t[b]];  // (cos, -sin)
+        e[b] = make_float2(fmaf(w.x, a.x, e[b].x), fmaf(w.x, a.y, e[b].y));
+        d[b] = make_float2(fmaf(-w.y, s.x, d[b].x), fmaf(-w.y, s.y, d[b].y));
+      }
+    }
+    if (c % 2 == 0) {
+      const float2 mid = x[(c / 2) << log];
+#pragma unroll
+      for (int b = 0; b < MB; ++b) {
+        const float sg = (m0 + b) & 1 ? -1.0f : 1.0f;
+        e[b] = make_float2(fmaf(sg, mid.x, e[b].x), fmaf(sg, mid.y, e[b].y));
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < MB; ++b) {
+      const int m = m0 + b;
+      if (m >= outs) break;
+      const float2 r = fftdev::rot<Fwd>(d[b]);
+      sink(line, k1 + f.r1 * m, cadd(e[b], r));
+      if (m > 0 && 2 * m != c) sink(line, k1 + f.r1 * (c - m), csub(e[b], r));
+    }
+  }
+}
+
+__device__ __forceinline__ void load_roots(const DctLine& f, float2* roots, const float2* __restrict__ twn) {
+  if (!f.direct) return;
+  for (int t = static_cast<int>(threadIdx.x); t < f.r2; t += kThreads) roots[t] = __ldg(twn + 2 * f.r1 * t);
+}
+
+// Pass 1 on rows y0 .. y0 + lines - 1.
+__device__ __forceinline__ void div_dctx_tile_two(const float* __restrict__ psi, float* __restrict__ d1, int ny,
+                                                  const DctLine& f, const float2* __restrict__ twn,
+                                                  const float2* __restrict__ dtw, int y0, float2* sm) {
+  if (!QHK_CHECK(f.rows_smem() <= debug::dynamic_smem_bytes() && y0 >= 0 && y0 < ny)) return;
+  const int n = f.n, h = f.h(), log = f.log_lines(), pn = f.pitch();
+  float2* xs = sm;
+  float2* zs = xs + f.area();
+  float2* roots = zs + f.area();
+  float* P = reinterpret_cast<float*>(roots + f.roots());  // rows y0 - 1 .. y0 + lines, then the output rows
+  const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
+  load_roots(f, roots, twn);
+  for (int rr = warp; rr < f.lines + 2; rr += kThreads / 32) {
+    const int y = y0 - 1 + rr;
+    const bool in = y >= 0 && y < ny;
+    for (int x = lane; x < n; x += 32) P[rr * pn + x] = in ? psi[static_cast<std::size_t>(y) * n + x] : 0.0f;
+  }
+  __syncthreads();
+  for (int i = static_cast<int>(threadIdx.x); i < (h << log); i += kThreads) {
+    const int row = i & (f.lines - 1), m = i >> log, y = y0 + row;
+    const float* c = P + (row + 1) * pn;
+    float r[2] = {0.0f, 0.0f};
+    if (y < ny) {
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const int x = makhoul_x(2 * m + b, n);
+        const float p = c[x];
+        float acc = 0.0f;
+        if (x + 1 < n) acc = __fadd_rn(acc, wrap_phase(__fsub_rn(c[x + 1], p)));
+        if (x > 0) acc = __fsub_rn(acc, wrap_phase(__fsub_rn(p, c[x - 1])));
+        if (y + 1 < ny) acc = __fadd_rn(acc, wrap_phase(__fsub_rn(c[x + pn], p)));
+        if (y > 0) acc = __fsub_rn(acc, wrap_phase(__fsub_rn(p, c[x - pn])));
+        r[b] = acc;
+      }
+    }
+    zs[i] = make_float2(r[0], r[1]);
+  }
+  __syncthreads();
+  dct_first<true>(f, xs, twn, [&](int line, int m) { return zs[(m << log) + line]; });
+  __syncthreads();
+  dct_second<true>(f, xs, roots, [&](int line, int k, float2 v) { zs[(k << log) + line] = v; });
+  __syncthreads();
+  for (int i = static_cast<int>(threadIdx.x); i < ((h + 1) << log); i += kThreads) {
+    const int row = i & (f.lines - 1), k = i >> log;
+    float xk, xnk;
+    dct_pair(zs + row, f.lines, k, h, twn, dtw, xk, xnk);
+    P[row * pn + k] = xk;
+    if (k > 0 && k < h) P[row * pn + n - k] = xnk;
+  }
+  __syncthreads();
+  for (int row = warp; row < f.lines && y0 + row < ny; row += kThreads / 32) {
+    for (int x = lane; x < n; x += 32) d1[static_cast<std::size_t>(y0 + row) * n + x] = P[row * pn + x];
+  }
+}
+
+// Pass 2 on columns c0 .. c0 + lines - 1 of an image of height f.n.
+__device__ __forceinline__ void dcty_solve_tile_two(const float* __restrict__ d1, float* __restrict__ d2, int nx,
+                                                    const DctLine& f, const float2* __restrict__ twn,
+                                                    const float2* __restrict__ dtw, const float* __restrict__ cos_y,
+                                                    const float* __restrict__ cos_x, int c0, float2* sm) {
+  if (!QHK_CHECK(f.cols_smem() <= debug::dynamic_smem_bytes() && c0 >= 0 && c0 < nx)) return;
+  const int n = f.n, h = f.h(), log = f.log_lines();
+  float2* xs = sm;
+  float2* zs = xs + f.area();
+  float2* roots = zs + f.area();
+  load_roots(f, roots, twn);
+  dct_first<true>(f, xs, twn, [&](int line, int m) {
+    const float* in = d1 + c0 + line;
+    return c0 + line < nx ? make_float2(in[static_cast<std::size_t>(makhoul_x(2 * m, n)) * nx],
+                                        in[static_cast<std::size_t>(makhoul_x(2 * m + 1, n)) * nx])
+                          : make_float2(0.0f, 0.0f);
+  });
+  __syncthreads();
+  dct_second<true>(f, xs, roots, [&](int line, int k, float2 v) { zs[(k << log) + line] = v; });
+  __syncthreads();
+  for (int i = static_cast<int>(threadIdx.x); i < ((h + 1) << log); i += kThreads) {
+    const int line = i & (f.lines - 1), k = i >> log, col = c0 + line;
+    const bool live = col < nx;
+    float xk, xnk;
+    dct_pair(zs + line, f.lines, k, h, twn, dtw, xk, xnk);
+    const float ex = __ldg(cos_x + (live ? col : 0));
+    float ak = 0.0f, ank = 0.0f;
+    if (live && !(k == 0 && col == 0)) ak = __fdiv_rn(xk, __fsub_rn(__fadd_rn(__ldg(cos_y + k), ex), 4.0f));
+    if (live && k > 0 && k < h) ank = __fdiv_rn(xnk, __fsub_rn(__fadd_rn(__ldg(cos_y + n - k), ex), 4.0f));
+    if (k == h) ank = ak;  // a[n - h] = a[h]
+    xs[i] = cmulc(make_float2(ak, k == 0 ? 0.0f : -ank), __ldg(dtw + k));  // A[k]
+  }
+  __syncthreads();
+  dct_first<false>(f, zs, twn, [&](int line, int k) {
+    return idct_merge(xs[(k << log) + line], xs[((h - k) << log) + line], k, twn);
+  });
+  __syncthreads();
+  const float inv = 1.0f / static_cast<float>(n);
+  dct_second<false>(f, zs, roots, [&](int line, int m, float2 v) {
+    if (c0 + line >= nx) return;
+    float* out = d2 + c0 + line;
+    out[static_cast<std::size_t>(makhoul_x(2 * m, n)) * nx] = v.x * inv;
+    out[static_cast<std::size_t>(makhoul_x(2 * m + 1, n)) * nx] = v.y * inv;
+  });
+}
+
+// Pass 3 on rows y0 .. y0 + lines - 1, in place, with the congruence partial sums (idctx_tile).
+__device__ __forceinline__ void idctx_tile_two(float* __restrict__ phi, const float* __restrict__ psi, int ny,
+                                               const DctLine& f, const float2* __restrict__ twn,
+                                               const float2* __restrict__ dtw, int y0, double* __restrict__ pair,
+                                               float2* sm, double (*red)[kThreads]) {
+  if (!QHK_CHECK(f.rows_smem() <= debug::dynamic_smem_bytes() && y0 >= 0 && y0 < ny)) return;
+  const int n = f.n, h = f.h(), log = f.log_lines(), pn = f.pitch();
+  float2* xs = sm;
+  float2* zs = xs + f.area();
+  float2* roots = zs + f.area();
+  float* F = reinterpret_cast<float*>(roots + f.roots());  // the spectral rows, then the image rows
+  const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  load_roots(f, roots, twn);
+  for (int row = warp; row < f.lines; row += kThreads / 32) {
+    const bool in = y0 + row < ny;
+    for (int x = lane; x < n; x += 32) F[row * pn + x] = in ? phi[static_cast<std::size_t>(y0 + row) * n + x] : 0.0f;
+  }
+  __syncthreads();
+  for (int i = tid; i < (h << log); i += kThreads) {
+    const int row = i & (f.lines - 1), k = i >> log;
+    const float* a = F + row * pn;
+    const float2 ak = cmulc(make_float2(a[k], k == 0 ? 0.0f : -a[n - k]), __ldg(dtw + k));
+    const float2 am = cmulc(make_float2(a[h - k], -a[h + k]), __ldg(dtw + h - k));  // k = 0: A[h], of which a[h] twice
+    zs[i] = idct_merge(ak, am, k, twn);
+  }
+  __syncthreads();
+  dct_first<false>(f, xs, twn, [&](int line, int k) { return zs[(k << log) + line]; });
+  __syncthreads();
+  const float inv = 1.0f / static_cast<float>(n);
+  dct_second<false>(f, xs, roots, [&](int line, int m, float2 v) {
+    F[line * pn + makhoul_x(2 * m, n)] = v.x * inv;
+    F[line * pn + makhoul_x(2 * m + 1, n)] = v.y * inv;
+  });
+  __syncthreads();
+  double sc = 0.0, ss = 0.0;
+  for (int row = warp; row < f.lines && y0 + row < ny; row += kThreads / 32) {
+    for (int x = lane; x < n; x += 32) {
+      const std::size_t g = static_cast<std::size_t>(y0 + row) * n + x;
+      const float v = F[row * pn + x];
+      phi[g] = v;
+      double s, c;
+      sincos(static_cast<double>(__fsub_rn(psi[g], v)), &s, &c);
+      sc += c;
+      ss += s;
+    }
+  }
+  red[0][tid] = sc;
+  red[1][tid] = ss;
+  __syncthreads();
+  for (int w = kThreads / 2; w > 0; w >>= 1) {
+    if (tid < w) {
+      red[0][tid] += red[0][tid + w];
+      red[1][tid] += red[1][tid + w];
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    pair[0] = red[0][0];
+    pair[1] = red[1][0];
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_div_dctx_two(const float* __restrict__ psi, float* __restrict__ d1, int ny, DctLine f,
+                   const float2* __restrict__ twn, const float2* __restrict__ dtw) {
+  extern __shared__ __align__(16) float2 sm[];
+  const std::size_t img = static_cast<std::size_t>(blockIdx.y) * ny * f.n;
+  div_dctx_tile_two(psi + img, d1 + img, ny, f, twn, dtw, static_cast<int>(blockIdx.x) * f.lines, sm);
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_dcty_solve_two(const float* __restrict__ d1, float* __restrict__ d2, int nx, DctLine f,
+                     const float2* __restrict__ twn, const float2* __restrict__ dtw,
+                     const float* __restrict__ cos_y, const float* __restrict__ cos_x) {
+  extern __shared__ __align__(16) float2 sm[];
+  const std::size_t img = static_cast<std::size_t>(blockIdx.y) * f.n * nx;
+  dcty_solve_tile_two(d1 + img, d2 + img, nx, f, twn, dtw, cos_y, cos_x, static_cast<int>(blockIdx.x) * f.lines, sm);
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_idctx_two(float* __restrict__ phi, const float* __restrict__ psi, int ny, DctLine f,
+                const float2* __restrict__ twn, const float2* __restrict__ dtw, double* __restrict__ partial) {
+  extern __shared__ __align__(16) float2 sm[];
+  __shared__ double red[2][kThreads];
+  const std::size_t img = static_cast<std::size_t>(blockIdx.y) * ny * f.n;
+  idctx_tile_two(phi + img, psi + img, ny, f, twn, dtw, static_cast<int>(blockIdx.x) * f.lines,
+                 partial + (static_cast<std::size_t>(blockIdx.y) * gridDim.x + blockIdx.x) * 2, sm, red);
+}
+
+// The three passes of a stack on this engine; false when it does not run lines of that length.
+bool pass1_two(const float* psi, float* d1, int count, int ny, int nx, const float2* twn, const float2* dtw,
+               cudaStream_t s) {
+  const DctLine f = dct_line(nx);
+  if (f.n == 0) return false;
+  ensure_smem(k_div_dctx_two);
+  k_div_dctx_two<<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(psi, d1, ny, f, twn, dtw);
+  check_launch("unwrap pass 1");
+  return true;
+}
+bool pass2_two(const float* d1, float* phi, int count, int ny, int nx, const float2* twn, const float2* dtw,
+               const float* cos_y, const float* cos_x, cudaStream_t s) {
+  const DctLine f = dct_line(ny);
+  if (f.n == 0) return false;
+  ensure_smem(k_dcty_solve_two);
+  k_dcty_solve_two<<<dim3((nx + f.lines - 1) / f.lines, count), kThreads, f.cols_smem(), s>>>(d1, phi, nx, f, twn, dtw,
+                                                                                              cos_y, cos_x);
+  check_launch("unwrap pass 2");
+  return true;
+}
+bool pass3_two(float* phi, const float* psi, int count, int ny, int nx, const float2* twn, const float2* dtw,
+               double* partial, cudaStream_t s) {
+  const DctLine f = dct_line(nx);
+  if (f.n == 0) return false;
+  ensure_smem(k_idctx_two);
+  k_idctx_two<<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(phi, psi, ny, f, twn, dtw,
+                                                                                         partial);
+  check_launch("unwrap pass 3");
+  return true;
+}
+
 // Rows of a pass-1 / pass-3 tile and columns of a pass-2 tile for lines of length n: the register
-// engine's R = 256 / T where it runs, else the staged tiles'. Every path (planned, batched, without
+// engine's R = 256 / T where it runs, the two-factor tiles' lines, else the staged tiles'. Every path (planned, batched, without
 // allocation) tiles alike, so that the congruence partial sums, and with them the results, agree.
 int rows_per_cta(int len, std::size_t extra_per_row);
 
 int unwrap_tile_rows(int nx) {
   const int t = unwrap_line_threads(nx);
-  return t ? kThreads / t : rows_per_cta(nx, static_cast<std::size_t>(nx) * sizeof(float));
+  if (t) return kThreads / t;
+  const DctLine l = dct_line(nx);
+  return l.n ? l.lines : rows_per_cta(nx, static_cast<std::size_t>(nx) * sizeof(float));
 }
 
 
@@ -766,7 +1140,7 @@ void UnwrapPlan::solve(const float* psi, float* phi, cudaStream_t s) {
     k_div_dctx_reg<T, V><<<dim3(nblk_, count_), kThreads, smem, s>>>(psi, d1_.get(), ny, Lx.tw, dtw_x_.get());
     check_launch("unwrap pass 1");
   });
-  if (!reg_rows) {
+  if (!reg_rows && !pass1_two(psi, d1_.get(), count_, ny, nx, Lx.tw, dtw_x_.get(), s)) {
     const std::size_t smem = 2 * static_cast<std::size_t>(nx) * (c + 1) * sizeof(float2) + (c + 2) * nx * sizeof(float);
     const dim3 grid(nblk_, count_);
 #define QHK_U1(C)                                                                                \
@@ -792,7 +1166,7 @@ void UnwrapPlan::solve(const float* psi, float* phi, cudaStream_t s) {
                                                         cos_x_.get());
     check_launch("unwrap pass 2");
   });
-  if (!reg_cols) {
+  if (!reg_cols && !pass2_two(d1_.get(), phi, count_, ny, nx, Ly.tw, dtw_y_.get(), cos_y_.get(), cos_x_.get(), s)) {
     int cc = 16;
     const auto smem_of = [&](int k) {
       return 2 * static_cast<std::size_t>(ny) * k * sizeof(float2) + static_cast<std::size_t>(ny) * k * sizeof(float);
@@ -823,7 +1197,7 @@ void UnwrapPlan::solve(const float* psi, float* phi, cudaStream_t s) {
       k_idctx_reg<T, V><<<dim3(nblk_, count_), kThreads, smem, s>>>(phi, psi, ny, Lx.tw, dtw_x_.get(), partial_.get());
       check_launch("unwrap pass 3");
     });
-  } else {
+  } else if (!pass3_two(phi, psi, count_, ny, nx, Lx.tw, dtw_x_.get(), partial_.get(), s)) {
     const std::size_t smem = 2 * static_cast<std::size_t>(nx) * (c + 1) * sizeof(float2) + c * nx * sizeof(float);
     const dim3 grid(nblk_, count_);
 #define QHK_U3(C)                                                                                    \
@@ -866,6 +1240,11 @@ void UnwrapPlan::rytov(const float* psi, const float* logamp, float* phi_scratch
 
 namespace {
 
+// Engines of a line length: each has launches of its own in a batch, so that each kernel holds only its own
+// tiles' registers.
+enum LineKind : int { kStaged = 0, kReg = 1, kTwo = 2 };
+int line_kind(int n) { return unwrap_line_threads(n) ? kReg : dct_line(n).n ? kTwo : kStaged; }
+
 // One image of an uneven batch, as the batch kernels see it.
 struct BatchImage {
   std::size_t offset;  // first pixel in the packed buffers
@@ -873,7 +1252,8 @@ struct BatchImage {
   int rows;            // rows per tile of passes 1 and 3 (as UnwrapPlan for this size)
   int cols;            // columns per tile of pass 2
   int nblk;            // row tiles
-  int reg_x, reg_y;    // rows (passes 1, 3) / columns (pass 2) on the register engine
+  int kind_x, kind_y;  // engine of the rows (passes 1, 3) and of the columns (pass 2)
+  DctLine line_x, line_y;  // their lines, where that is kTwo
   int partial;         // first congruence partial pair of this image
   FftLen Lx, Ly;
   const float2* dtw_x;
@@ -935,8 +1315,8 @@ __device__ __forceinline__ int next_item(int* counter) {
     default: CALL(1); break;     \
   }
 
-template <bool Reg>
-__global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
+template <int Kind>
+__global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     k_batch_pass1(const float* __restrict__ psi, float* __restrict__ d1, const BatchQueue Q) {
   extern __shared__ __align__(16) float2 sm[];
   for (int it = next_item(Q.counter); it < Q.n; it = next_item(Q.counter)) {
@@ -946,8 +1326,10 @@ __global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
 #define QHK_R1(T, V)                                                                                      \
   div_dctx_tile_reg<T, V>(psi + im.offset, d1 + im.offset, im.ny, im.Lx.tw, im.dtw_x, w.y * (kThreads / T), sm)
 #define QHK_P1(C) div_dctx_tile<C>(psi + im.offset, d1 + im.offset, im.ny, im.nx, im.Lx, im.dtw_x, w.y * (C), sm)
-    if constexpr (Reg) {
+    if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.nx, QHK_R1)
+    } else if constexpr (Kind == kTwo) {
+      div_dctx_tile_two(psi + im.offset, d1 + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, sm);
     } else {
       QHK_ROWS_SWITCH(im.rows, QHK_P1)
     }
@@ -957,8 +1339,8 @@ __global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
   }
 }
 
-template <bool Reg>
-__global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
+template <int Kind>
+__global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     k_batch_pass2(const float* __restrict__ d1, float* __restrict__ phi, const BatchQueue Q) {
   extern __shared__ __align__(16) float2 sm[];
   for (int it = next_item(Q.counter); it < Q.n; it = next_item(Q.counter)) {
@@ -971,8 +1353,11 @@ __global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
 #define QHK_P2(C)                                                                                                  \
   dcty_solve_tile<C>(d1 + im.offset, phi + im.offset, im.ny, im.nx, im.Ly, im.dtw_y, im.cos_y, im.cos_x, w.y * (C), \
                      sm)
-    if constexpr (Reg) {
+    if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.ny, QHK_R2)
+    } else if constexpr (Kind == kTwo) {
+      dcty_solve_tile_two(d1 + im.offset, phi + im.offset, im.nx, im.line_y, im.Ly.tw, im.dtw_y, im.cos_y, im.cos_x,
+                          w.y * im.line_y.lines, sm);
     } else {
       QHK_ROWS_SWITCH(im.cols, QHK_P2)
     }
@@ -982,8 +1367,8 @@ __global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
   }
 }
 
-template <bool Reg>
-__global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
+template <int Kind>
+__global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     k_batch_pass3(float* __restrict__ phi, const float* __restrict__ psi, double* __restrict__ partial,
                   const BatchQueue Q) {
   extern __shared__ __align__(16) float2 sm[];
@@ -997,8 +1382,11 @@ __global__ void __launch_bounds__(kThreads, Reg ? 2 : 1)
   idctx_tile_reg<T, V>(phi + im.offset, psi + im.offset, im.ny, im.Lx.tw, im.dtw_x, w.y * (kThreads / T), pair, sm, red)
 #define QHK_P3(C) \
   idctx_tile<C>(phi + im.offset, psi + im.offset, im.ny, im.nx, im.Lx, im.dtw_x, w.y * (C), pair, sm, red)
-    if constexpr (Reg) {
+    if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.nx, QHK_R3)
+    } else if constexpr (Kind == kTwo) {
+      idctx_tile_two(phi + im.offset, psi + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, pair,
+                     sm, red);
     } else {
       QHK_ROWS_SWITCH(im.rows, QHK_P3)
     }
@@ -1064,6 +1452,13 @@ __global__ void __launch_bounds__(kThreads)
 #undef QHK_ROWS_SWITCH
 #undef QHK_REG_SWITCH
 
+template <class F>
+void with_kinds(F&& f) {
+  f.template operator()<kStaged>();
+  f.template operator()<kReg>();
+  f.template operator()<kTwo>();
+}
+
 int solve_cols(int ny) {
   int cc = 16;
   const auto smem_of = [&](int k) {
@@ -1106,7 +1501,7 @@ UnwrapBatchPlan::UnwrapBatchPlan(const int* ny, const int* nx, int count) {
     return side[n];
   };
   int partial = 0;
-  std::size_t smem[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  std::size_t smem[kBatchPasses] = {};
   for (int i = 0; i < count; ++i) {
     require(ny[i] >= 2 && nx[i] >= 2 && ny[i] % 2 == 0 && nx[i] % 2 == 0, "unwrap: image sides must be even");
     BatchImage& b = im[i];
@@ -1115,10 +1510,14 @@ UnwrapBatchPlan::UnwrapBatchPlan(const int* ny, const int* nx, int count) {
     total_ += static_cast<std::size_t>(ny[i]) * nx[i];
     b.ny = ny[i];
     b.nx = nx[i];
-    b.reg_x = unwrap_line_threads(b.nx) != 0;
-    b.reg_y = unwrap_line_threads(b.ny) != 0;
+    b.kind_x = line_kind(b.nx);
+    b.kind_y = line_kind(b.ny);
+    b.line_x = dct_line(b.nx);
+    b.line_y = dct_line(b.ny);
     b.rows = unwrap_tile_rows(b.nx);
-    b.cols = b.reg_y ? kThreads / unwrap_line_threads(b.ny) : solve_cols(b.ny);
+    b.cols = b.kind_y == kReg   ? kThreads / unwrap_line_threads(b.ny)
+             : b.kind_y == kTwo ? b.line_y.lines
+                                : solve_cols(b.ny);
     b.nblk = (b.ny + b.rows - 1) / b.rows;
     b.partial = partial;
     partial += b.nblk;
@@ -1130,18 +1529,28 @@ UnwrapBatchPlan::UnwrapBatchPlan(const int* ny, const int* nx, int count) {
     b.dtw_y = dtw_[ty].get();
     b.cos_y = cos_[ty].get();
     const std::size_t row_buf = 2 * static_cast<std::size_t>(b.nx) * (b.rows + 1) * sizeof(float2);
-    if (!with_unwrap_line(b.nx, [&]<int T, int V>() {
-          smem[5] = std::max(smem[5], reg_rows_smem<T, V>());
-          smem[7] = std::max(smem[7], reg_rows_smem<T, V>());
-        })) {
-      smem[0] = std::max(smem[0], row_buf + (b.rows + 2) * static_cast<std::size_t>(b.nx) * sizeof(float));
-      smem[2] = std::max(smem[2], row_buf + b.rows * static_cast<std::size_t>(b.nx) * sizeof(float));
+    const int px = 3 * b.kind_x, py = 3 * b.kind_y;  // passes 1, 2, 3 of a kind at 3 kind + 0, 1, 2
+    if (b.kind_x == kReg) {
+      with_unwrap_line(b.nx, [&]<int T, int V>() {
+        smem[px] = std::max(smem[px], reg_rows_smem<T, V>());
+        smem[px + 2] = std::max(smem[px + 2], reg_rows_smem<T, V>());
+      });
+    } else if (b.kind_x == kTwo) {
+      smem[px] = std::max(smem[px], b.line_x.rows_smem());
+      smem[px + 2] = std::max(smem[px + 2], b.line_x.rows_smem());
+    } else {
+      smem[px] = std::max(smem[px], row_buf + (b.rows + 2) * static_cast<std::size_t>(b.nx) * sizeof(float));
+      smem[px + 2] = std::max(smem[px + 2], row_buf + b.rows * static_cast<std::size_t>(b.nx) * sizeof(float));
     }
-    if (!with_unwrap_line(b.ny, [&]<int T, int V>() { smem[6] = std::max(smem[6], reg_cols_smem<T, V>()); })) {
-      smem[1] = std::max(smem[1], 2 * static_cast<std::size_t>(b.ny) * b.cols * sizeof(float2) +
-                                      static_cast<std::size_t>(b.ny) * b.cols * sizeof(float));
+    if (b.kind_y == kReg) {
+      with_unwrap_line(b.ny, [&]<int T, int V>() { smem[py + 1] = std::max(smem[py + 1], reg_cols_smem<T, V>()); });
+    } else if (b.kind_y == kTwo) {
+      smem[py + 1] = std::max(smem[py + 1], b.line_y.cols_smem());
+    } else {
+      smem[py + 1] = std::max(smem[py + 1], 2 * static_cast<std::size_t>(b.ny) * b.cols * sizeof(float2) +
+                                                static_cast<std::size_t>(b.ny) * b.cols * sizeof(float));
     }
-    smem[3] = std::max(smem[3], static_cast<std::size_t>(b.nx + b.ny) * sizeof(float));
+    smem[kConstsPass] = std::max(smem[kConstsPass], static_cast<std::size_t>(b.nx + b.ny) * sizeof(float));
   }
   // Items, largest images first so that the queue ends with small tiles.
   std::vector<int> order(count);
@@ -1149,20 +1558,19 @@ UnwrapBatchPlan::UnwrapBatchPlan(const int* ny, const int* nx, int count) {
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
     return static_cast<std::size_t>(im[a].ny) * im[a].nx > static_cast<std::size_t>(im[b].ny) * im[b].nx;
   });
-  std::vector<int2> items[8];
+  std::vector<int2> items[kBatchPasses];
   for (const int i : order) {
     const BatchImage& b = im[i];
-    for (int t = 0; t < b.nblk; ++t) items[b.reg_x ? 5 : 0].push_back(make_int2(i, t));
-    for (int t = 0; t < (b.nx + b.cols - 1) / b.cols; ++t) items[b.reg_y ? 6 : 1].push_back(make_int2(i, t));
-    items[3].push_back(make_int2(i, 0));
+    for (int t = 0; t < b.nblk; ++t) items[3 * b.kind_x].push_back(make_int2(i, t));
+    for (int t = 0; t < (b.nx + b.cols - 1) / b.cols; ++t) items[3 * b.kind_y + 1].push_back(make_int2(i, t));
+    items[kConstsPass].push_back(make_int2(i, 0));
     const std::size_t pixels = static_cast<std::size_t>(b.ny) * b.nx;
-    for (std::size_t t = 0; t * kAssembleChunk < pixels; ++t) items[4].push_back(make_int2(i, static_cast<int>(t)));
+    for (std::size_t t = 0; t * kAssembleChunk < pixels; ++t) items[kConstsPass + 1].push_back(make_int2(i, static_cast<int>(t)));
   }
-  items[2] = items[0];
-  items[7] = items[5];
+  for (const int kind : {kStaged, kReg, kTwo}) items[3 * kind + 2] = items[3 * kind];
   std::vector<int2> all;
-  std::size_t at[8];
-  for (int p = 0; p < 8; ++p) {
+  std::size_t at[kBatchPasses];
+  for (int p = 0; p < kBatchPasses; ++p) {
     at[p] = all.size();
     all.insert(all.end(), items[p].begin(), items[p].end());
   }
@@ -1170,23 +1578,22 @@ UnwrapBatchPlan::UnwrapBatchPlan(const int* ny, const int* nx, int count) {
   check(cudaMemcpy(items_.get(), all.data(), all.size() * sizeof(int2), cudaMemcpyHostToDevice), "upload items");
   images_.reset(count * sizeof(BatchImage));
   check(cudaMemcpy(images_.get(), im.data(), count * sizeof(BatchImage), cudaMemcpyHostToDevice), "upload images");
-  counters_.reset(8);
+  counters_.reset(kBatchPasses);
   d1_.reset(total_);
   partial_.reset(2 * static_cast<std::size_t>(partial));
   consts_.reset(count);
-  for (int p = 0; p < 8; ++p) {
+  for (int p = 0; p < kBatchPasses; ++p) {
     pass_[p].items = items_.get() + at[p];
     pass_[p].n = static_cast<int>(items[p].size());
     pass_[p].smem = smem[p];
   }
-  pass_[0].grid = persistent_grid(k_batch_pass1<false>, smem[0], pass_[0].n);
-  pass_[1].grid = persistent_grid(k_batch_pass2<false>, smem[1], pass_[1].n);
-  pass_[2].grid = persistent_grid(k_batch_pass3<false>, smem[2], pass_[2].n);
-  pass_[5].grid = persistent_grid(k_batch_pass1<true>, smem[5], pass_[5].n);
-  pass_[6].grid = persistent_grid(k_batch_pass2<true>, smem[6], pass_[6].n);
-  pass_[7].grid = persistent_grid(k_batch_pass3<true>, smem[7], pass_[7].n);
-  pass_[3].grid = persistent_grid(k_batch_pass4, smem[3], pass_[3].n);
-  pass_[4].grid = persistent_grid(k_batch_pass5, 0, pass_[4].n);
+  with_kinds([&]<int Kind>() {
+    pass_[3 * Kind].grid = persistent_grid(k_batch_pass1<Kind>, smem[3 * Kind], pass_[3 * Kind].n);
+    pass_[3 * Kind + 1].grid = persistent_grid(k_batch_pass2<Kind>, smem[3 * Kind + 1], pass_[3 * Kind + 1].n);
+    pass_[3 * Kind + 2].grid = persistent_grid(k_batch_pass3<Kind>, smem[3 * Kind + 2], pass_[3 * Kind + 2].n);
+  });
+  pass_[kConstsPass].grid = persistent_grid(k_batch_pass4, smem[kConstsPass], pass_[kConstsPass].n);
+  pass_[kConstsPass + 1].grid = persistent_grid(k_batch_pass5, 0, pass_[kConstsPass + 1].n);
 }
 
 UnwrapBatchPlan::~UnwrapBatchPlan() = default;
@@ -1206,42 +1613,30 @@ void UnwrapBatchPlan::unwrap(const float* psi, float* phi, cudaStream_t s) {
   const auto queue = [&](int p) {
     return BatchQueue{imgs, static_cast<const int2*>(pass_[p].items), pass_[p].n, count(), total_, q + p};
   };
-  check(cudaMemsetAsync(q, 0, 8 * sizeof(int), s), "cudaMemset");
-  // Each of passes 1-3 runs as up to two persistent launches: the images whose lines the register engine
-  // takes (pass_[5 + p]) and the others (pass_[p]).
-  for (const bool reg : {false, true}) {
-    const int p = reg ? 5 : 0;
-    if (pass_[p].n == 0) continue;
-    if (reg) {
-      k_batch_pass1<true><<<pass_[p].grid, kThreads, pass_[p].smem, s>>>(psi, d1_.get(), queue(p));
-    } else {
-      k_batch_pass1<false><<<pass_[p].grid, kThreads, pass_[p].smem, s>>>(psi, d1_.get(), queue(p));
-    }
+  check(cudaMemsetAsync(q, 0, kBatchPasses * sizeof(int), s), "cudaMemset");
+  // Each of passes 1-3 runs as up to three persistent launches, one per engine that some image's lines take.
+  with_kinds([&]<int Kind>() {
+    const Pass& p = pass_[3 * Kind];
+    if (p.n == 0) return;
+    k_batch_pass1<Kind><<<p.grid, kThreads, p.smem, s>>>(psi, d1_.get(), queue(3 * Kind));
     check_launch("unwrap batch pass 1");
-  }
-  for (const bool reg : {false, true}) {
-    const int p = reg ? 6 : 1;
-    if (pass_[p].n == 0) continue;
-    if (reg) {
-      k_batch_pass2<true><<<pass_[p].grid, kThreads, pass_[p].smem, s>>>(d1_.get(), phi, queue(p));
-    } else {
-      k_batch_pass2<false><<<pass_[p].grid, kThreads, pass_[p].smem, s>>>(d1_.get(), phi, queue(p));
-    }
+  });
+  with_kinds([&]<int Kind>() {
+    const Pass& p = pass_[3 * Kind + 1];
+    if (p.n == 0) return;
+    k_batch_pass2<Kind><<<p.grid, kThreads, p.smem, s>>>(d1_.get(), phi, queue(3 * Kind + 1));
     check_launch("unwrap batch pass 2");
-  }
-  for (const bool reg : {false, true}) {
-    const int p = reg ? 7 : 2;
-    if (pass_[p].n == 0) continue;
-    if (reg) {
-      k_batch_pass3<true><<<pass_[p].grid, kThreads, pass_[p].smem, s>>>(phi, psi, partial_.get(), queue(p));
-    } else {
-      k_batch_pass3<false><<<pass_[p].grid, kThreads, pass_[p].smem, s>>>(phi, psi, partial_.get(), queue(p));
-    }
+  });
+  with_kinds([&]<int Kind>() {
+    const Pass& p = pass_[3 * Kind + 2];
+    if (p.n == 0) return;
+    k_batch_pass3<Kind><<<p.grid, kThreads, p.smem, s>>>(phi, psi, partial_.get(), queue(3 * Kind + 2));
     check_launch("unwrap batch pass 3");
-  }
-  k_batch_pass4<<<pass_[3].grid, kThreads, pass_[3].smem, s>>>(phi, partial_.get(), consts_.get(), queue(3));
+  });
+  const Pass& consts = pass_[kConstsPass];
+  k_batch_pass4<<<consts.grid, kThreads, consts.smem, s>>>(phi, partial_.get(), consts_.get(), queue(kConstsPass));
   check_launch("unwrap batch constants");
-  k_batch_pass5<<<pass_[4].grid, kThreads, 0, s>>>(phi, consts_.get(), queue(4));
+  k_batch_pass5<<<pass_[kConstsPass + 1].grid, kThreads, 0, s>>>(phi, consts_.get(), queue(kConstsPass + 1));
   check_launch("unwrap batch constant");
 }
 
@@ -1357,7 +1752,7 @@ void unwrap_noalloc(const float* psi, float* phi, int count, int ny, int nx, cud
     k_div_dctx_reg<T, V><<<dim3(nblk, count), kThreads, reg_rows_smem<T, V>(), s>>>(psi, d1, ny, fft_x, dtw_x);
     check_launch("unwrap_noalloc pass 1");
   });
-  if (!reg_rows) {
+  if (!reg_rows && !pass1_two(psi, d1, count, ny, nx, fft_x, dtw_x, s)) {
     const std::size_t smem = 2 * static_cast<std::size_t>(nx) * (rows + 1) * sizeof(float2) + (rows + 2) * nx * sizeof(float);
     const dim3 grid(nblk, count);
 #define QHK_S1(C)                                                                   \
@@ -1381,7 +1776,7 @@ void unwrap_noalloc(const float* psi, float* phi, int count, int ny, int nx, cud
     k_dcty_solve_reg<T, V><<<grid, kThreads, reg_cols_smem<T, V>(), s>>>(d1, phi, nx, fft_y, dtw_y, cos_y, cos_x);
     check_launch("unwrap_noalloc pass 2");
   });
-  if (!reg_cols) {
+  if (!reg_cols && !pass2_two(d1, phi, count, ny, nx, fft_y, dtw_y, cos_y, cos_x, s)) {
     int cc = 16;
     const auto smem_of = [&](int k) {
       return 2 * static_cast<std::size_t>(ny) * k * sizeof(float2) + static_cast<std::size_t>(ny) * k * sizeof(float);
@@ -1410,7 +1805,7 @@ void unwrap_noalloc(const float* psi, float* phi, int count, int ny, int nx, cud
       k_idctx_reg<T, V><<<dim3(nblk, count), kThreads, reg_rows_smem<T, V>(), s>>>(phi, psi, ny, fft_x, dtw_x, partial);
       check_launch("unwrap_noalloc pass 3");
     });
-  } else {
+  } else if (!pass3_two(phi, psi, count, ny, nx, fft_x, dtw_x, partial, s)) {
     const std::size_t smem = 2 * static_cast<std::size_t>(nx) * (rows + 1) * sizeof(float2) + rows * nx * sizeof(float);
     const dim3 grid(nblk, count);
 #define QHK_S3(C)                                                                              \

@@ -73,9 +73,10 @@ class UnwrapBatchPlan {
   DevBuf<float> d1_;
   DevBuf<double> partial_;
   DevBuf<float2> consts_;
-  // Passes 1-5 (staged tiles for passes 1-3), then passes 1-3 of the images whose lines run on the
-  // register engine: each has its own queue, so that each kernel holds only its own tiles' registers.
-  Pass pass_[8];
+  // Passes 1-3 of the images whose lines run on the staged, the register and the two-factor engine (each a
+  // queue of its own, so that each kernel holds only its own tiles' registers), then passes 4 and 5.
+  static constexpr int kConstsPass = 9, kBatchPasses = 11;
+  Pass pass_[kBatchPasses];
   CapturedWork graph_;
   bool warmed_ = false;
 };
