@@ -609,8 +609,11 @@ struct Fgp2Args {
   float* pout[3];       // p_{k+2}
   float* rout[3];       // r_{k+2} (not written when step k + 1 is the last)
   int nz, ny, nx;
-  int pitch;  // shared-memory row length: nx rounded up to 32 floats (the box width)
+  int pitch;  // shared-memory row length: the tile's width rounded up to 32 floats (the box width)
   int ytiles;
+  // Tiles over x (k_fgp2's Window form): each computes `win` columns from xt inner - 4 on (from 0 on and all of
+  // nx when xtiles is 1) and writes columns xt inner .. (xt + 1) inner - 1.
+  int xtiles, inner, win;
   float lambda, step;
   float m1, m2;     // momenta of steps k and k + 1
   float neg_zero;  // -0.0f, the addend of the packed products (a value the compiler cannot see)
@@ -713,18 +716,28 @@ __device__ __forceinline__ void fgp_dual_pair(float2 c, float2 cz, float2 cy, fl
 // x value (ceil(threads / pitch)).
 constexpr std::size_t fgp2_rows(int ty) { return 20 * static_cast<std::size_t>(ty) + 64; }
 // Threads per CTA the two-step kernel is compiled for (nx / 4 x TY must stay within it).
-constexpr int fgp2_threads(int ty) { return ty == 8 ? 512 : 256; }
+constexpr int fgp2_threads(int ty) { return ty >= 8 ? 512 : 256; }
 
 // CUBE > 0: compiled for a CUBE^3 volume (the sizes, the pitch and the block shape are constants, so
 // shared-memory and global addresses fold into immediate offsets); 0: any size, from the arguments.
-template <int TY, bool FIRST, bool LAST, int CUBE = 0>
+//
+// Window: tiles over x as well, for rows that do not fit one tile (two steps of 160 x 300 x 320 in 244 us, two
+// one-step passes 317), and taller tiles of shorter rows, up to what 512 threads and the shared memory hold:
+// fewer halo rows and planes run ahead, against more work between the barriers of a plane (150 x 180^2, a
+// middle pair of steps: 85 us with 11 rows, 81 with 8, the last pair 62 and 72; the tuner picks). A window's
+// results depend on the two columns beside it per side (one per step, and the shifted x differences), so it
+// computes four more columns on each side than it writes: what the outermost of them lack is not written,
+// and the box loads' x stays on 16 bytes.
+template <int TY, bool FIRST, bool LAST, int CUBE = 0, bool Window = false>
 __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const __grid_constant__ Fgp2Maps M) {
   extern __shared__ __align__(128) float smem2[];
   constexpr int VEC = 4;
   constexpr int RK_ROWS = TY + 4, B_ROWS = TY + 3, R1_ROWS = TY + 2, Z1_ROWS = TY + 1;
   constexpr int HALO = (8 + TY - 1) / TY;  // halo pair slots per thread: 2 nx over nx / 4 * TY threads
   constexpr bool kFullWarps = CUBE > 0 && (CUBE / VEC * TY) % 32 == 0;
-  const int nx = CUBE > 0 ? CUBE : A.nx, ny = CUBE > 0 ? CUBE : A.ny, nz = CUBE > 0 ? CUBE : A.nz;
+  // nx: columns of the tile; nxg: of the volume.
+  const int nx = CUBE > 0 ? CUBE : Window ? A.win : A.nx, ny = CUBE > 0 ? CUBE : A.ny, nz = CUBE > 0 ? CUBE : A.nz;
+  const int nxg = CUBE > 0 ? CUBE : A.nx;
   const int bx = CUBE > 0 ? CUBE / VEC : static_cast<int>(blockDim.x);
   const int tx = static_cast<int>(threadIdx.x);
   const int ty = static_cast<int>(threadIdx.y);
@@ -734,7 +747,7 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
   const int lane = linear & 31;
   const int warp_threads = kFullWarps ? 32 : min(32, nthreads - (linear & ~31));
   const unsigned lanes = warp_threads >= 32 ? 0xffffffffu : ((1u << warp_threads) - 1u);
-  const std::size_t nxy = static_cast<std::size_t>(nx) * ny;
+  const std::size_t nxy = static_cast<std::size_t>(nxg) * ny;
   // Shared memory in floats, rows of P floats (A.pitch: nx rounded up to 128 bytes; the columns
   // from nx on hold the zeros the box loads fill in): slot strides and buffer bases (32-bit offsets
   // from smem2), then the mbarriers. r_{k+1} keeps in shared memory only what other threads read:
@@ -754,8 +767,10 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
   const int own_b = (ty + 1) * P + x0;
   const int own_z1 = ty * P + x0;
   // The thread's four own points run as two pairs of packed operations; x guards per point.
-  const bool x_first = x0 == 0;       // point 0 is x = 0
-  const bool x_last = x0 + VEC == nx;  // point 3 is x = nx - 1
+  int xg0 = 0;                    // the tile's first column in the volume
+  bool x_first = x0 == 0;         // point 0 is x = 0
+  bool x_last = x0 + VEC == nxg;  // point 3 is x = nx - 1
+  bool x_own = true;              // the tile writes this thread's columns
   const auto f2 = [](float a, float b) { return make_float2(a, b); };
   const float2 nzero = make_float2(A.neg_zero, A.neg_zero);
   // Primal points of the own row of plane z (y given); left = x component of the dual at x0-1.
@@ -850,18 +865,26 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
   const auto ld2 = [](const float* p) { return *reinterpret_cast<const float2*>(p); };
   const auto st2 = [](float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; };
 
-  const long long units = static_cast<long long>(CUBE > 0 ? (CUBE + TY - 1) / TY : A.ytiles) * nz;
+  const long long units = static_cast<long long>(CUBE > 0 ? (CUBE + TY - 1) / TY : Window ? A.ytiles * A.xtiles : A.ytiles) * nz;
   const long long u_end = units * (blockIdx.x + 1) / gridDim.x;
   for (long long u = units * blockIdx.x / gridDim.x; u < u_end;) {
-    const int y0 = static_cast<int>(u / nz) * TY;
+    const int tile = static_cast<int>(u / nz);
+    const int xt = Window ? tile / A.ytiles : 0;
+    const int y0 = (tile - xt * A.ytiles) * TY;
     const int z0 = static_cast<int>(u % nz);
     if (!QHK_CHECK(y0 < ny && u < units)) break;  // CTA-uniform
+    if constexpr (Window) {
+      xg0 = A.xtiles > 1 ? xt * A.inner - 4 : 0;
+      x_first = xg0 + x0 == 0;
+      x_last = xg0 + x0 + VEC == nxg;
+      x_own = xg0 + x0 >= xt * A.inner && xg0 + x0 < min((xt + 1) * A.inner, nxg);
+    }
     const int zend = static_cast<int>(min(static_cast<long long>(nz), z0 + (u_end - u)));
     u += zend - z0;
     const int zmax = min(zend + 1, nz - 1);  // last plane of r_k and b read
     const int y = y0 + ty;
     const bool own = y < ny;
-    const std::size_t own_g = static_cast<std::size_t>(y) * nx + x0;  // within a plane
+    const std::size_t own_g = static_cast<std::size_t>(y) * nxg + (xg0 + x0);  // within a plane
 
     // Box loads by thread 0, counted on an mbarrier. A plane z into ring slot s (z mod 3): r_k rows
     // y0-2 .. y0+TY+1 (`comps` components) and b rows y0-1 .. y0+TY+1, on mbarrier s; p_k of plane
@@ -873,15 +896,15 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
       std::uint64_t* bar = bars + s;
       arm(s);
       tma::mbar_expect(bar, static_cast<unsigned>((comps * RK_ROWS + (with_b ? B_ROWS : 0)) * P * 4));
-      for (int c = 0; c < comps; ++c) tma::load_3d(smem2 + (s * 3 + c) * RKP, &M.r[c], 0, y0 - 2, z, bar);
-      if (with_b) tma::load_3d(smem2 + OB + s * BP, &M.b, 0, y0 - 1, z, bar);
+      for (int c = 0; c < comps; ++c) tma::load_3d(smem2 + (s * 3 + c) * RKP, &M.r[c], xg0, y0 - 2, z, bar);
+      if (with_b) tma::load_3d(smem2 + OB + s * BP, &M.b, xg0, y0 - 1, z, bar);
     };
     const auto issue_pk = [&](int z) {
       if (!QHK_CHECK(z >= 0 && z < nz)) return;
       tma::fence_async_shared();
       arm(3);
       tma::mbar_expect(bars + 3, static_cast<unsigned>(3 * R1_ROWS * P * 4));
-      for (int c = 0; c < 3; ++c) tma::load_3d(smem2 + OPK + c * R1P, &M.p[c], 0, y0 - 1, z, bars + 3);
+      for (int c = 0; c < 3; ++c) tma::load_3d(smem2 + OPK + c * R1P, &M.p[c], xg0, y0 - 1, z, bars + 3);
     };
     // Bounded wait on mbarrier i (every thread), then its phase bit flips.
     const auto wait_bar = [&](int i) {
@@ -957,7 +980,7 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
           if (side >= 0 && side <= 2 && yy >= 0 && yy < ny) {
             const int i = (zi + 1) * P + x;  // r_k row of yy
             const float2 vx = ld2(Rx + i);
-            const float2 o = fgp_primal_pair(a < nz - 1, a > 0, yy < ny - 1, yy > 0, x == 0, x + 1 == nx - 1,
+            const float2 o = fgp_primal_pair(a < nz - 1, a > 0, yy < ny - 1, yy > 0, xg0 + x == 0, xg0 + x + 1 == nxg - 1,
                                              ld2(Rz + i), ld2(Rzb + i), ld2(Ry + i), ld2(Ry + i - P), vx,
                                              f2(x > 0 ? Rx[i - 1] : 0.0f, vx.x), ld2(B + zi * P + x), A.lambda, nzero);
             st2(Z + zi * P + x, o);
@@ -1025,7 +1048,7 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
               r[c] = ld2(R + c * RKP + i + P);
               p[c] = FIRST ? r[c] : ld2(PK + c * R1P + i);
             }
-            fgp_dual_pair(c0, cz, cy, cx, a < nz - 1, yy < ny - 1, x + 1 == nx - 1, A.step, A.m1, p, r, nzero);
+            fgp_dual_pair(c0, cz, cy, cx, a < nz - 1, yy < ny - 1, xg0 + x + 1 == nxg - 1, A.step, A.m1, p, r, nzero);
             st2(Ry1 + i, r[1]);
             if (side == 1) {
               st2(RzH + x, r[0]);
@@ -1071,7 +1094,7 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
             if (hz_side[j] == 3) {
               const int i = (TY + 1) * P + x;
               const float2 vx = ld2(RxH + x);
-              const float2 o = fgp_primal_pair(a < nz - 1, a > 0, yy < ny - 1, yy > 0, x == 0, x + 1 == nx - 1,
+              const float2 o = fgp_primal_pair(a < nz - 1, a > 0, yy < ny - 1, yy > 0, xg0 + x == 0, xg0 + x + 1 == nxg - 1,
                                                ld2(RzH + x), ld2(RzbH + x), ld2(Ry + i), ld2(Ry + i - P), vx,
                                                f2(x > 0 ? RxH[x - 1] : 0.0f, vx.x), ld2(B + i), A.lambda, nzero);
               st2(Z + TY * P + x, o);
@@ -1089,11 +1112,13 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
         const float right = (x0 + VEC < nx && (lane == 31 || lane == warp_threads - 1)) ? Zc[own_z1 + VEC] : from_lane;
         if (own) {
           dual4(q, y, zc, zn, zy, right, A.m2, cp, cr);
-          const std::size_t at = q * nxy + own_g;
+          if (!Window || x_own) {
+            const std::size_t at = q * nxy + own_g;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            Vec<VEC>::store(A.pout[c] + at, cp[c]);
-            if (!LAST) Vec<VEC>::store(A.rout[c] + at, cr[c]);
+            for (int c = 0; c < 3; ++c) {
+              Vec<VEC>::store(A.pout[c] + at, cp[c]);
+              if (!LAST) Vec<VEC>::store(A.rout[c] + at, cr[c]);
+            }
           }
         }
       }
@@ -1116,7 +1141,10 @@ struct FgpShape {
   int ty;
   int grid;
   std::size_t smem;
-  int variant = 0;  // 0: r stored (k_fgp), 1: r recomputed (k_fgp_p), 2: two steps per pass (k_fgp2)
+  int variant = 0;  // 0: r stored (k_fgp), 1: r recomputed (k_fgp_p), 2: two steps per pass (k_fgp2),
+                    // 3: two steps per pass in windows
+  int xtiles = 1, inner = 0, win = 0;  // of variant 3
+  [[nodiscard]] bool two_step() const { return variant >= 2; }
 };
 
 // Shared memory of the two-step form (rows of the 128-byte-aligned pitch, then 3 mbarriers), and
@@ -1134,6 +1162,42 @@ bool fgp2_fits(int nx, int ty) {
   return nx % 4 == 0 && nx <= 256 && (nx / 4) * ty <= fgp2_threads(ty) && fgp2_smem(nx, ty) <= kSmemOptin;
 }
 
+// The window form's tiles: the rows of a volume in `xtiles` windows of `win` columns, `ty` rows tall.
+struct Fgp2Window {
+  int ty = 0, xtiles = 0, inner = 0, win = 0;
+};
+constexpr int kWindowRows[] = {16, 14, 12, 11, 10, 8};  // instantiated heights
+constexpr int kMaxWindows = 8;
+// The tallest tile with `xtiles` windows; ty = 0 when none fits.
+Fgp2Window fgp2_window(int nx, int xtiles) {
+  Fgp2Window w;
+  if (nx % 4 != 0) return w;
+  w.xtiles = xtiles;
+  w.inner = xtiles == 1 ? nx : ((nx + xtiles - 1) / xtiles + 3) / 4 * 4;
+  w.win = xtiles == 1 ? nx : w.inner + 8;
+  if ((xtiles - 1) * w.inner >= nx) return w;  // an empty window
+  for (const int ty : kWindowRows) {
+    if (fgp2_fits(w.win, ty)) {
+      w.ty = ty;
+      break;
+    }
+  }
+  return w;
+}
+// The windows that give the fewest tiles over a plane (a march's planes take about the same time whatever the
+// tile), fewer windows on ties; ty = 0 when none fits.
+Fgp2Window fgp2_fewest_tiles(int ny, int nx) {
+  Fgp2Window best;
+  int tiles = 0;
+  for (int t = 1; t <= kMaxWindows; ++t) {
+    const Fgp2Window w = fgp2_window(nx, t);
+    if (w.ty == 0) continue;
+    const int n = t * ((ny + w.ty - 1) / w.ty);
+    if (best.ty == 0 || n < tiles) best = w, tiles = n;
+  }
+  return best;
+}
+
 // Shared memory of the r-recomputing step: 3 ring slots + 1 staging plane of 3 components x TY + 2
 // rows, 2 primal and 2 b planes of TY + 1 rows (no staging on the first step).
 std::size_t fgp_p_smem(int nx, int ty, bool first) {
@@ -1141,7 +1205,7 @@ std::size_t fgp_p_smem(int nx, int ty, bool first) {
          sizeof(float);
 }
 
-// Autotuner choices: variant * 16 + rows per CTA.
+// Autotuner choices: variant * 16 + rows per CTA; for the window form, variant * 16 + number of windows.
 constexpr int kFgpVariantScale = 16;
 
 std::size_t fgp_smem(int nx, int ty) {
@@ -1159,6 +1223,10 @@ std::vector<int> fgp_rows_candidates(int nx, bool two_step) {
   if (VEC == 4 && two_step) {
     for (const int ty : {8, 4, 2})
       if (fgp2_fits(nx, ty)) out.push_back(2 * kFgpVariantScale + ty);
+    for (int t = 1; t <= kMaxWindows; ++t) {
+      const Fgp2Window w = fgp2_window(nx, t);
+      if (w.ty > (t == 1 ? 8 : 7)) out.push_back(3 * kFgpVariantScale + t);
+    }
   }
   for (const int variant : {1, 0}) {
     for (const int ty : {8, 4, 2, 1}) {
@@ -1184,10 +1252,36 @@ TuneKey fgp_key(int nz, int ny, int nx) {
   return tune_key(TuneFamily::fgp, {nz, ny, nx, VEC, 0, 0});
 }
 
+// Calls f.template operator()<TY>() for a height of the window form.
+template <class F>
+void with_window_rows(int ty, F&& f) {
+  switch (ty) {
+    case 16: f.template operator()<16>(); break;
+    case 14: f.template operator()<14>(); break;
+    case 12: f.template operator()<12>(); break;
+    case 11: f.template operator()<11>(); break;
+    case 10: f.template operator()<10>(); break;
+    default: f.template operator()<8>(); break;
+  }
+}
+
 template <int VEC>
 FgpShape fgp_shape_rows(int nz, int ny, int nx, int choice) {
   const int variant = choice / kFgpVariantScale;
   const int ty = choice % kFgpVariantScale;
+  if (variant == 3) {
+    const Fgp2Window w = fgp2_window(nx, ty);
+    const std::size_t smem = fgp2_smem(w.win, w.ty);
+    const long long units = static_cast<long long>((ny + w.ty - 1) / w.ty) * w.xtiles * nz;
+    int per_sm = 0;
+    with_window_rows(w.ty, [&]<int TY>() {
+      auto kernel = k_fgp2<TY, false, false, 0, true>;
+      ensure_smem(kernel);
+      check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, (w.win / 4) * TY, smem), "cudaOccupancy");
+    });
+    const long long slots = static_cast<long long>(sm_count()) * std::max(per_sm, 1);
+    return FgpShape{w.ty, static_cast<int>(std::min(slots, units)), smem, 3, w.xtiles, w.inner, w.win};
+  }
   const std::size_t smem =
       variant == 2 ? fgp2_smem(nx, ty) : variant == 1 ? fgp_p_smem(nx, ty, false) : fgp_smem(nx, ty);
   int per_sm = 0;
@@ -1228,24 +1322,25 @@ template <int VEC>
 FgpShape fgp_shape(int nz, int ny, int nx, bool two_step) {
   const int form = g_fgp_form.load();
   const int fallback = fgp_rows_default<VEC>(nx);
-  int choice = tuned_choice(fgp_key<VEC>(nz, ny, nx), fallback);
+  // Untuned, two steps per pass with the fewest tiles where the caller's buffers allow it (160 x 300 x 320, ten
+  // steps: 1.13 ms, in two windows of 11 rows, where the stored-r form took 1.56), else the stored-r form.
+  const Fgp2Window fewest = VEC == 4 && two_step ? fgp2_fewest_tiles(ny, nx) : Fgp2Window{};
+  const int two = fewest.ty == 0                             ? fallback
+                  : fewest.xtiles == 1 && fewest.ty == 8 ? 2 * kFgpVariantScale + 8
+                                                         : 3 * kFgpVariantScale + fewest.xtiles;
+  int choice = tuned_choice(fgp_key<VEC>(nz, ny, nx), two);
   if (form == 3) {
-    choice = fallback;
-    for (const int ty : {8, 4, 2}) {
-      if (fgp2_fits(nx, ty)) {
-        choice = 2 * kFgpVariantScale + ty;
-        break;
-      }
-    }
+    choice = two;
   } else if (form >= 16) {  // two steps per pass with form - 16 rows, where that fits
     choice = fgp2_fits(nx, form - 16) ? 2 * kFgpVariantScale + (form - 16) : fallback;
   } else if (form == 1 || form == 2) {
-    const int ty = choice / kFgpVariantScale == 2 ? fallback : choice % kFgpVariantScale;
+    const int ty = choice / kFgpVariantScale >= 2 ? fallback : choice % kFgpVariantScale;
     choice = (form - 1) * kFgpVariantScale + ty;
     const std::size_t smem = form == 2 ? fgp_p_smem(nx, ty, false) : fgp_smem(nx, ty);
     if (smem > 200 * 1024) choice = (form - 1) * kFgpVariantScale + 1;
   }
-  if (choice / kFgpVariantScale == 2 && (VEC != 4 || !two_step || !fgp2_fits(nx, choice % kFgpVariantScale))) {
+  const int variant = choice / kFgpVariantScale, of = choice % kFgpVariantScale;
+  if (variant >= 2 && (VEC != 4 || !two_step || (variant == 2 ? !fgp2_fits(nx, of) : of < 1 || fgp2_window(nx, of).ty == 0))) {
     choice = fallback;
   }
   return fgp_shape_rows<VEC>(nz, ny, nx, choice);
@@ -1271,38 +1366,46 @@ void launch_fgp_p(const FgpPArgs& a, const FgpShape& sh, cudaStream_t s) {
   check_launch("fgp step");
 }
 
-template <int TY, bool FIRST, bool LAST, int CUBE>
+template <int TY, bool FIRST, bool LAST, int CUBE, bool Window>
 void launch_fgp2_t(const Fgp2Args& a, const float* const rin[3], const float* b, int grid, cudaStream_t s) {
-  auto kernel = k_fgp2<TY, FIRST, LAST, CUBE>;
+  auto kernel = k_fgp2<TY, FIRST, LAST, CUBE, Window>;
   ensure_smem(kernel);
   Fgp2Maps maps;
   for (int c = 0; c < 3; ++c) maps.r[c] = volume_tensor_map(rin[c], a.nx, a.ny, a.nz, a.pitch, TY + 4);
   maps.b = volume_tensor_map(b, a.nx, a.ny, a.nz, a.pitch, TY + 3);
   for (int c = 0; c < 3; ++c) maps.p[c] = FIRST ? maps.r[c] : volume_tensor_map(a.pin[c], a.nx, a.ny, a.nz, a.pitch, TY + 2);
-  kernel<<<grid, dim3(a.nx / 4, TY), fgp2_smem(a.nx, TY), s>>>(a, maps);
+  const int width = Window ? a.win : a.nx;
+  kernel<<<grid, dim3(width / 4, TY), fgp2_smem(width, TY), s>>>(a, maps);
   check_launch("fgp two steps");
 }
 
-template <int TY, int CUBE = 0>
+template <int TY, int CUBE = 0, bool Window = false>
 void launch_fgp2_rows(bool first, bool last, const Fgp2Args& a, const float* const rin[3], const float* b, int grid,
                       cudaStream_t s) {
   if (first && last) {
-    launch_fgp2_t<TY, true, true, CUBE>(a, rin, b, grid, s);
+    launch_fgp2_t<TY, true, true, CUBE, Window>(a, rin, b, grid, s);
   } else if (first) {
-    launch_fgp2_t<TY, true, false, CUBE>(a, rin, b, grid, s);
+    launch_fgp2_t<TY, true, false, CUBE, Window>(a, rin, b, grid, s);
   } else if (last) {
-    launch_fgp2_t<TY, false, true, CUBE>(a, rin, b, grid, s);
+    launch_fgp2_t<TY, false, true, CUBE, Window>(a, rin, b, grid, s);
   } else {
-    launch_fgp2_t<TY, false, false, CUBE>(a, rin, b, grid, s);
+    launch_fgp2_t<TY, false, false, CUBE, Window>(a, rin, b, grid, s);
   }
 }
 
 // rin: r_k (p_0 on the first step), b: the point the prox is taken at.
 void launch_fgp2(bool first, bool last, Fgp2Args a, const float* const rin[3], const float* b, const FgpShape& sh,
                  cudaStream_t s) {
+  a.neg_zero = -0.0f;
+  if (sh.variant == 3) {
+    require(fgp2_fits(sh.win, sh.ty), "tv: two-step FGP shape out of range");
+    a.pitch = fgp2_pitch(sh.win);
+    a.xtiles = sh.xtiles, a.inner = sh.inner, a.win = sh.win;
+    with_window_rows(sh.ty, [&]<int TY>() { launch_fgp2_rows<TY, 0, true>(first, last, a, rin, b, sh.grid, s); });
+    return;
+  }
   require(fgp2_fits(a.nx, sh.ty), "tv: two-step FGP shape out of range");
   a.pitch = fgp2_pitch(a.nx);
-  a.neg_zero = -0.0f;
   if (sh.ty == 8 && a.nx == 256 && a.ny == 256 && a.nz == 256) {  // the 256^3 volumes, sizes compiled in
     launch_fgp2_rows<8, 256>(first, last, a, rin, b, sh.grid, s);
   } else if (sh.ty == 8) {
@@ -1389,7 +1492,7 @@ void tv_prox(const float* b, TvBuffers& t, int nz, int ny, int nx, float lambda,
   const FgpShape sh = vec == 4 ? fgp_shape<4>(nz, ny, nx, t.has_fourth()) : fgp_shape<1>(nz, ny, nx, false);
   const float step = 1.0f / (12.0f * lambda);
   float tk = 1.0f;
-  if (sh.variant != 2 && t.p_index == 3) {
+  if (!sh.two_step() && t.p_index == 3) {
     // The one-step forms rotate among the first three triplets: bring p there (only after the form
     // changed between two calls on the same buffers).
     const std::size_t vbytes = static_cast<std::size_t>(nz) * ny * nx * sizeof(float);
@@ -1397,7 +1500,7 @@ void tv_prox(const float* b, TvBuffers& t, int nz, int ny, int nx, float lambda,
       check(cudaMemcpyAsync(t.v[0][c], t.v[3][c], vbytes, cudaMemcpyDeviceToDevice, s), "copy dual");
     t.p_index = 0;
   }
-  if (sh.variant == 2) {
+  if (sh.two_step()) {
     // Pairs of steps: (p, r) in two triplets -> (p, r) in two others; the first pair reads p_0 as
     // r_0. An odd last step runs the one-step kernel (stored-r form of the same shape family).
     int pc = t.p_index, rc = t.p_index;
@@ -1568,7 +1671,7 @@ void tune_fgp_rows(float* b, TvBuffers& t, int nz, int ny, int nx, float lambda,
   autotune(fgp_key<VEC>(nz, ny, nx), fgp_rows_candidates<VEC>(nx, t.has_fourth()), fgp_rows_default<VEC>(nx),
            [&](int choice) {
              const FgpShape sh = fgp_shape_rows<VEC>(nz, ny, nx, choice);
-             if (sh.variant == 2) {
+             if (sh.two_step()) {
                w.ytiles = (ny + sh.ty - 1) / sh.ty;
                launch_fgp2(false, false, w, w_rin, b, sh, s);
              } else if (sh.variant == 1) {
