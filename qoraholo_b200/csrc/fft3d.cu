@@ -737,7 +737,12 @@ void axis_pass(float2* data, int n_outer, std::size_t so, int n, std::size_t sp,
   } else if (axis_reg_variants(n) > 0 && radix_tuning_enabled()) {
     engine = tuned_choice(engine_key(n_outer, so, n, sp, ni, forward, mode, batch), 1);
   }
-  if (engine != 0 && axis_pass_reg(data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb, engine)) {
+  // 192 and 512 on the register engine hold 24 and 32 values a thread; without the restore the two-factor engine is
+  // faster (192^3: y pass 12 us against 17; 512^3: 208 against 296, from_data 265 against 317; with it 23 against
+  // 21 and 527 against 512).
+  const bool restore = mode == AxisMode::restore_half || mode == AxisMode::restore_mask;
+  const bool two = forced < 0 && (n == 192 || n == 512) && !restore && axis_two_covers(n) && !radix_tuning_enabled();
+  if (!two && engine != 0 && axis_pass_reg(data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb, engine)) {
     return;
   }
   if (engine != 0 && axis_two_covers(n)) {

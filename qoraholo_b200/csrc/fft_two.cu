@@ -1,5 +1,5 @@
 // FFT passes on the two-factor line transforms (fft_two.cuh): axis passes (tiles of columns) and row
-// passes (real rows transformed two at a time) for every length that is a product of two radices, at most
+// passes (real rows as half-length lines) for every length that is a product of two radices, at most
 // 16 and at most 32. The first DFT of a line takes its values straight from global memory and the last one
 // stores straight to it, so a transform costs one exchange through shared memory, where the staged engine
 // (fft_engine.cuh) goes through it once per radix pass and twice more for the load and the store.
@@ -7,11 +7,11 @@
 // What bounds these passes is HBM (or L2) latency and bandwidth: a tile's loads are all issued at once
 // (16 to 32 per thread) and several CTAs share an SM, so one CTA's loads overlap another's transforms.
 // Measured on B200 against the staged passes: half spectrum of 384^3, y pass 96 us (4.7 TB/s) from 171, z pass
-// with the restore 225 us from 321; of 8 x 96^3, y 13 us from 32, z 25 us from 61; complex rows of 97 x 384^2
+// with the restore 205 us from 321; of 8 x 96^3, y 13 us from 32, z 22 us from 61; complex rows of 97 x 384^2
 // 53 us from 97. Lengths with a compile-time form on the register engine (fft_reg.cu) stay there: 256^3 y 27 us
-// against 30 here, z 53 against 63, C2R rows 31 against 39, and 384-long C2R-R2C rows 156 against 237.
+// against 30 here, z 53 against 63.
 #include "debug.cuh"
-#include "fft_two.cuh"
+#include "fft_rows.cuh"
 #include "fft_two.hpp"
 
 namespace qhk {
@@ -19,10 +19,16 @@ namespace qhk {
 namespace {
 
 using twofft::Factors;
+using twofft::row_launch;
+using twofft::row_line_pitch;
+using twofft::row_tile;
+using twofft::RowLaunch;
+using twofft::RowTile;
 
 // CTAs per SM to leave registers for, at 256 threads each (axis tiles are 16 columns of at most 16 threads or 8
 // columns of at most 32, row tiles 256 threads): three of 80 registers where the radices fit them, two of 128
-// for larger radices and for the restore, whose two transforms spill at 80 (96^3 x 8: 25 us against 29).
+// for larger radices and for the restore, whose two transforms spill at 80 (96^3 x 8: 25 us against 29); the
+// restore of second factors up to 24 in three CTAs of 192 threads.
 constexpr int min_blocks(int max) { return max == twofft::kSmall ? 3 : 2; }
 
 constexpr bool restores(int mode) {
@@ -33,7 +39,8 @@ constexpr bool restores(int mode) {
 
 // COLS = 1 << logc consecutive columns of one outer slice per CTA; COLS * R2 threads (R2 >= R1).
 template <bool Fwd, int Mode, int Max>
-__global__ void __launch_bounds__(256, restores(Mode) ? 2 : min_blocks(Max))
+__global__ void __launch_bounds__(restores(Mode) && Max == twofft::kMid ? 192 : 256,
+                                  !restores(Mode) ? min_blocks(Max) : Max == twofft::kMid ? 3 : 2)
     k_axis_two(float2* __restrict__ data, std::size_t so, std::size_t sp, int ni, Factors f, int logc,
                const float2* __restrict__ tw, float scale, const float2* __restrict__ aux_a,
                const std::uint8_t* __restrict__ aux_h, std::size_t sb) {
@@ -170,141 +177,111 @@ void axis_two_mode(const Factors& f, int cols, float2* data, int n_outer, std::s
 }
 
 // ---- real rows <-> half spectra -----------------------------------------------------------------------
-// Two consecutive rows a, b make one complex line a + i b of the full length nx, so that the spectrum pair
-// and the line are related by sums alone: Z[k] = A[k] + i B[k], Z[nx - k] = conj A[k] + i conj B[k], and the
-// real rows are the line's real and imaginary parts. A tile is `lines` pairs, f.r2 threads each.
+// A row of nx = 2 M real values as M complex values (the pairs 2m, 2m + 1) through a length-M transform, with
+// the split and merge formulas of the staged rows (fft3d.cu). A tile is `lines` rows, f.r2 threads each.
 
-// Slots of a tile of rows: consecutive threads are consecutive j of a line (first pass) or consecutive k1
-// (second pass), so B = 1 and A is odd; lines are C apart, with C congruent to the number of threads per
-// line modulo the 16 two-bank slots where a half-warp spans several lines.
-__host__ __device__ __forceinline__ int row_line_pitch(const Factors& f) {
-  const int need = f.r1 * (f.r2 | 1);
-  const int want = f.r2 < 16 ? f.r2 : f.r1;
-  return need + ((want - need) % 16 + 16) % 16;
+// Value m of the length-M line whose inverse transform gives the pairs of a row, from its half spectrum.
+__device__ __forceinline__ float2 merge_value(const float2* __restrict__ e_row, int m, int M,
+                                              const float2* __restrict__ twn) {
+  float2 a = e_row[m], b = e_row[M - m];
+  if (m == 0) a.y = b.y = 0.0f;  // a real signal has real bins 0 and M; their imaginary parts drop out
+  const float2 sv = make_float2(a.x + b.x, a.y - b.y);  // a + conj(b)
+  const float2 d = make_float2(a.x - b.x, a.y + b.y);   // a - conj(b)
+  const float2 t = cmulc(d, __ldg(twn + m));             // d e^{2 pi i m / nx}
+  return make_float2(sv.x - t.y, sv.y + t.x);            // sv + i t
 }
 
-// Position k of the line a + i b from the half spectra of the two rows; imaginary parts of the real bins
-// 0 and nx / 2 drop out.
-__device__ __forceinline__ float2 pair_value(const float2* __restrict__ ea, const float2* __restrict__ eb, bool both,
-                                             int k, int n) {
-  const int h = n / 2;
-  const int kk = k <= h ? k : n - k;
-  float2 a = ea[kk];
-  float2 b = both ? eb[kk] : make_float2(0.0f, 0.0f);
-  if (kk == 0 || kk == h) a.y = b.y = 0.0f;
-  return k <= h ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, b.x - a.y);
-}
-
-// Rows of the pairs in `zs` (natural order, n + 1 apart) to their half spectra, one warp per pair at a time.
-__device__ __forceinline__ void split_pairs(const float2* zs, int n, std::size_t line0, int lines, std::size_t rows,
-                                            float2* __restrict__ e) {
-  const int h = n / 2 + 1;
+// Lines in `zs` (natural order, M + 1 apart) to their rows' half spectra, one warp per row at a time.
+__device__ __forceinline__ void split_rows(const float2* zs, int M, std::size_t row0, int lines, std::size_t rows,
+                                           const float2* __restrict__ twn, float2* __restrict__ e) {
   const int warps = static_cast<int>(blockDim.x + 31) >> 5;
-  for (int l = static_cast<int>(threadIdx.x) >> 5; l < lines; l += warps) {
-    const std::size_t row = 2 * (line0 + l);
-    if (row >= rows) break;
-    const float2* z = zs + l * (n + 1);
-    float2* ea = e + row * h;
-    const bool both = row + 1 < rows;
-    for (int k = static_cast<int>(threadIdx.x) & 31; k < h; k += 32) {
-      const float2 zk = z[k], zm = z[k == 0 ? 0 : n - k];
-      ea[k] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-      if (both) ea[h + k] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+  for (int l = static_cast<int>(threadIdx.x) >> 5; l < lines && row0 + l < rows; l += warps) {
+    const float2* z = zs + l * (M + 1);
+    float2* out = e + (row0 + l) * (M + 1);
+    for (int k = static_cast<int>(threadIdx.x) & 31; k <= M; k += 32) {
+      const float2 zk = z[k == M ? 0 : k], zm = z[k == 0 ? 0 : M - k];
+      const float2 ev = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+      const float2 od = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));  // (zk - conj zm) / 2i
+      out[k] = cadd(ev, cmul(__ldg(twn + k), od));
     }
   }
 }
 
-// The threads of the last warp beyond lines * R2 only take part in split_pairs and the barriers.
-struct RowTile {
-  int line, j;      // first pass: line and butterfly
-  int line2, j2;    // second pass
-  bool first, second;
-};
-__device__ __forceinline__ RowTile row_tile(const Factors& f, int lines) {
-  RowTile r;
-  const int t = static_cast<int>(threadIdx.x);
-  r.line = t / f.r2;
-  r.j = t - r.line * f.r2;
-  r.first = r.line < lines;
-  r.line2 = t / f.r1;
-  r.j2 = t - r.line2 * f.r1;
-  r.second = r.line2 < lines;
-  return r;
-}
-
-template <bool Clamp, int Max>
-__global__ void __launch_bounds__(256, min_blocks(Max))
-    k_rows_r2c_two(const float* __restrict__ x, float2* __restrict__ e, std::size_t rows, Factors f, int lines,
-                   const float2* __restrict__ tw) {
-  extern __shared__ float2 xs[];
-  const int n = f.n(), A = f.r2 | 1, C = row_line_pitch(f);
-  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + n + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
-  float2* zs = xs + lines * C;
-  const std::size_t line0 = static_cast<std::size_t>(blockIdx.x) * lines;
-  const RowTile r = row_tile(f, lines);
-  if (r.first) {
-    const std::size_t row = 2 * (line0 + r.line);
-    const bool la = row < rows, lb = row + 1 < rows;
-    twofft::with_first<Max>(f.r1, [&]<int R>() {
-      float2 v[R];
-      const float* p = x + (la ? row * n : 0) + r.j;
-#pragma unroll
-      for (int q = 0; q < R; ++q, p += f.r2) {
-        v[q] = make_float2(la ? p[0] : 0.0f, lb ? p[n] : 0.0f);
-        if (Clamp) v[q] = make_float2(fmaxf(v[q].x, 0.0f), fmaxf(v[q].y, 0.0f));
-      }
-      twofft::first_pass<R, true>(v, r.j, tw, xs + r.line * C + r.j, A);
-    });
-  }
+// Second pass of a forward transform into natural order, and the split.
+template <int Max>
+__device__ __forceinline__ void finish_r2c(const Factors& f, const RowTile& r, const float2* xs, int C, float2* zs,
+                                           std::size_t row0, int lines, std::size_t rows,
+                                           const float2* __restrict__ twn, float2* __restrict__ e) {
+  const int M = f.n(), A = f.r2 | 1;
   __syncthreads();
   if (r.second) {
     twofft::with_radix<Max>(f.r2, [&]<int R>() {
       float2 u[R];
       twofft::second_pass<R, true>(u, xs + r.line2 * C + r.j2 * A, 1);
 #pragma unroll
-      for (int q = 0; q < R; ++q) zs[r.line2 * (n + 1) + r.j2 + f.r1 * q] = u[q];
+      for (int q = 0; q < R; ++q) zs[r.line2 * (M + 1) + r.j2 + f.r1 * q] = u[q];
     });
   }
   __syncthreads();
-  split_pairs(zs, n, line0, lines, rows, e);
+  split_rows(zs, M, row0, lines, rows, twn, e);
+}
+
+template <bool Clamp, int Max>
+__global__ void __launch_bounds__(256, min_blocks(Max))
+    k_rows_r2c_two(const float* __restrict__ x, float2* __restrict__ e, std::size_t rows, Factors f, int lines,
+                   const float2* __restrict__ tw, const float2* __restrict__ twn) {
+  extern __shared__ float2 xs[];
+  const int M = f.n(), A = f.r2 | 1, C = row_line_pitch(f);
+  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + M + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
+  const std::size_t row0 = static_cast<std::size_t>(blockIdx.x) * lines;
+  const RowTile r = row_tile(f, lines);
+  if (r.first) {
+    const bool live = row0 + r.line < rows;
+    twofft::with_first<Max>(f.r1, [&]<int R>() {
+      float2 v[R];
+      const float2* p = reinterpret_cast<const float2*>(x) + (live ? row0 + r.line : 0) * M + r.j;
+#pragma unroll
+      for (int q = 0; q < R; ++q, p += f.r2) {
+        v[q] = live ? *p : make_float2(0.0f, 0.0f);
+        if (Clamp) v[q] = make_float2(fmaxf(v[q].x, 0.0f), fmaxf(v[q].y, 0.0f));
+      }
+      twofft::first_pass<R, true>(v, r.j, tw, xs + r.line * C + r.j, A);
+    });
+  }
+  finish_r2c<Max>(f, r, xs, C, xs + lines * C, row0, lines, rows, twn, e);
 }
 
 template <int Mode, int Max>
 __global__ void __launch_bounds__(256, min_blocks(Max))
     k_rows_c2r_two(const float2* __restrict__ e, float* __restrict__ x, std::size_t rows, Factors f, int lines,
-                   const float2* __restrict__ tw, float nm2, float inv_k02) {
+                   const float2* __restrict__ tw, const float2* __restrict__ twn, float nm2, float inv_k02) {
   extern __shared__ float2 xs[];
-  const int n = f.n(), h = n / 2 + 1, A = f.r2 | 1, C = row_line_pitch(f);
+  const int M = f.n(), A = f.r2 | 1, C = row_line_pitch(f);
   if (!QHK_CHECK(static_cast<std::size_t>(lines) * C * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
-  const std::size_t line0 = static_cast<std::size_t>(blockIdx.x) * lines;
+  const std::size_t row0 = static_cast<std::size_t>(blockIdx.x) * lines;
   const RowTile r = row_tile(f, lines);
   if (r.first) {
-    const std::size_t row = 2 * (line0 + r.line);
-    const bool la = row < rows, lb = row + 1 < rows;
-    const float2* ea = e + (la ? row : 0) * h;
+    const float2* er = e + (row0 + r.line < rows ? row0 + r.line : 0) * (M + 1);
     twofft::with_first<Max>(f.r1, [&]<int R>() {
       float2 v[R];
 #pragma unroll
-      for (int q = 0; q < R; ++q) v[q] = pair_value(ea, ea + h, lb, r.j + q * f.r2, n);
+      for (int q = 0; q < R; ++q) v[q] = merge_value(er, r.j + q * f.r2, M, twn);
       twofft::first_pass<R, false>(v, r.j, tw, xs + r.line * C + r.j, A);
     });
   }
   __syncthreads();
-  const std::size_t row = 2 * (line0 + r.line2);
-  if (r.second && row < rows) {
-    const bool lb = row + 1 < rows;
+  if (r.second && row0 + r.line2 < rows) {
     twofft::with_radix<Max>(f.r2, [&]<int R>() {
       float2 u[R];
       twofft::second_pass<R, false>(u, xs + r.line2 * C + r.j2 * A, 1);
-      float* p = x + row * n + r.j2;
+      float2* p = reinterpret_cast<float2*>(x) + (row0 + r.line2) * M + r.j2;
 #pragma unroll
       for (int q = 0; q < R; ++q, p += f.r1) {
         float2 z = u[q];
         if (Mode == static_cast<int>(C2rMode::index)) {
           z = make_float2(index_from_potential(z.x, 0.0f, nm2, inv_k02), index_from_potential(z.y, 0.0f, nm2, inv_k02));
         }
-        p[0] = z.x;
-        if (lb) p[n] = z.y;
+        *p = z;
       }
     });
   }
@@ -314,21 +291,20 @@ __global__ void __launch_bounds__(256, min_blocks(Max))
 // second pass of the inverse and the first of the forward transform, on values one thread holds.
 template <int Max>
 __global__ void __launch_bounds__(256, min_blocks(Max))
-    k_rows_c2r_r2c_two(float2* __restrict__ e, std::size_t rows, Factors f, int lines, const float2* __restrict__ tw) {
+    k_rows_c2r_r2c_two(float2* __restrict__ e, std::size_t rows, Factors f, int lines, const float2* __restrict__ tw,
+                       const float2* __restrict__ twn) {
   extern __shared__ float2 xs[];
-  const int n = f.n(), h = n / 2 + 1, A = f.r2 | 1, C = row_line_pitch(f);
-  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + n + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
+  const int M = f.n(), A = f.r2 | 1, C = row_line_pitch(f);
+  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + M + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
   float2* zs = xs + lines * C;
-  const std::size_t line0 = static_cast<std::size_t>(blockIdx.x) * lines;
+  const std::size_t row0 = static_cast<std::size_t>(blockIdx.x) * lines;
   const RowTile r = row_tile(f, lines);
   if (r.first) {
-    const std::size_t row = 2 * (line0 + r.line);
-    const bool la = row < rows, lb = row + 1 < rows;
-    const float2* ea = e + (la ? row : 0) * h;
+    const float2* er = e + (row0 + r.line < rows ? row0 + r.line : 0) * (M + 1);
     twofft::with_first<Max>(f.r1, [&]<int R>() {
       float2 v[R];
 #pragma unroll
-      for (int q = 0; q < R; ++q) v[q] = pair_value(ea, ea + h, lb, r.j + q * f.r2, n);
+      for (int q = 0; q < R; ++q) v[q] = merge_value(er, r.j + q * f.r2, M, twn);
       twofft::first_pass<R, false>(v, r.j, tw, xs + r.line * C + r.j, A);
     });
   }
@@ -349,37 +325,33 @@ __global__ void __launch_bounds__(256, min_blocks(Max))
       float2 v[R];
       twofft::second_pass<R, true>(v, xs + r.line * C + r.j, A);
 #pragma unroll
-      for (int q = 0; q < R; ++q) zs[r.line * (n + 1) + r.j + f.r2 * q] = v[q];
+      for (int q = 0; q < R; ++q) zs[r.line * (M + 1) + r.j + f.r2 * q] = v[q];
     });
   }
   __syncthreads();
-  split_pairs(zs, n, line0, lines, rows, e);
+  split_rows(zs, M, row0, lines, rows, twn, e);
 }
 
 // The end of one FISTA-TV iteration and the start of the next on rows (fft3d.cu k_rows_tv_final_r2c: the
 // final primal, the momentum point, xprev, and the R2C of the momentum point), with the same operations;
-// the momentum point is formed with row-contiguous loads into shared memory, one warp per row at a time, and
-// rows pair up in the transform. 256^3: 93 us (470 MB, 5.0 TB/s) from 109; 150 x 180^2: 34 us from 48.
+// the momentum point is formed with row-contiguous loads into shared memory, one warp per row at a time, 256^3: 93 us (470 MB, 5.0 TB/s) from 109; 150 x 180^2: 34 us from 48.
 template <int Max>
 __global__ void __launch_bounds__(256, min_blocks(Max))
     k_rows_tv_final_r2c_two(const float* __restrict__ b, const float* __restrict__ pz, const float* __restrict__ py,
                             const float* __restrict__ px, int nz, int ny, float lambda, float momentum,
                             float* __restrict__ xprev, float2* __restrict__ e, std::size_t rows, Factors f, int lines,
-                            const float2* __restrict__ tw) {
+                            const float2* __restrict__ tw, const float2* __restrict__ twn) {
   extern __shared__ float2 xs[];
-  const int n = f.n(), A = f.r2 | 1, C = row_line_pitch(f);
-  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + n + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
-  float2* zs = xs + lines * C;
-  float* ys = reinterpret_cast<float*>(zs);  // the real rows before the transform, n apart
-  const std::size_t line0 = static_cast<std::size_t>(blockIdx.x) * lines;
+  const int M = f.n(), n = 2 * M, A = f.r2 | 1, C = row_line_pitch(f);
+  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + M + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
+  float2* zs = xs + lines * C;  // the pairs of the momentum point's rows (M + 1 apart), then the spectrum
+  const std::size_t row0 = static_cast<std::size_t>(blockIdx.x) * lines;
   const std::size_t nxy = static_cast<std::size_t>(n) * ny;
-  const int M = n / 2;
   {
     const int warps = static_cast<int>(blockDim.x + 31) >> 5;
-    const std::size_t row0 = 2 * line0;
-    const int nr = static_cast<int>(min(static_cast<std::size_t>(2 * lines), rows - min(row0, rows)));
-    for (int w = static_cast<int>(threadIdx.x) >> 5; w < 2 * lines; w += warps) {
-      float2* yrow = reinterpret_cast<float2*>(ys + w * n);
+    const int nr = static_cast<int>(min(static_cast<std::size_t>(lines), rows - min(row0, rows)));
+    for (int w = static_cast<int>(threadIdx.x) >> 5; w < lines; w += warps) {
+      float2* yrow = zs + w * (M + 1);
       if (w >= nr) {
         for (int m = static_cast<int>(threadIdx.x) & 31; m < M; m += 32) yrow[m] = make_float2(0.0f, 0.0f);
         continue;
@@ -424,23 +396,13 @@ __global__ void __launch_bounds__(256, min_blocks(Max))
   if (r.first) {
     twofft::with_first<Max>(f.r1, [&]<int R>() {
       float2 v[R];
-      const float* p = ys + 2 * r.line * n + r.j;
+      const float2* p = zs + r.line * (M + 1) + r.j;
 #pragma unroll
-      for (int q = 0; q < R; ++q, p += f.r2) v[q] = make_float2(p[0], p[n]);
+      for (int q = 0; q < R; ++q, p += f.r2) v[q] = *p;
       twofft::first_pass<R, true>(v, r.j, tw, xs + r.line * C + r.j, A);
     });
   }
-  __syncthreads();
-  if (r.second) {
-    twofft::with_radix<Max>(f.r2, [&]<int R>() {
-      float2 u[R];
-      twofft::second_pass<R, true>(u, xs + r.line2 * C + r.j2 * A, 1);
-#pragma unroll
-      for (int q = 0; q < R; ++q) zs[r.line2 * (n + 1) + r.j2 + f.r1 * q] = u[q];
-    });
-  }
-  __syncthreads();
-  split_pairs(zs, n, line0, lines, rows, e);
+  finish_r2c<Max>(f, r, xs, C, zs, row0, lines, rows, twn, e);
 }
 
 // ---- complex rows -------------------------------------------------------------------------------------
@@ -503,28 +465,6 @@ __global__ void __launch_bounds__(256, min_blocks(Max))
   }
 }
 
-// Lines per CTA: about 256 threads, within 64 KB of shared memory.
-int lines_per_cta(const Factors& f, bool staged) {
-  const std::size_t line = (row_line_pitch(f) + (staged ? f.n() + 1 : 0)) * sizeof(float2);
-  int lines = 256 / f.r2;
-  while (lines > 1 && lines * line > 64 * 1024) --lines;
-  return lines;
-}
-
-struct RowLaunch {
-  int lines, threads;
-  std::size_t smem;
-  unsigned grid;
-};
-RowLaunch row_launch(const Factors& f, std::size_t total_lines, bool staged) {
-  RowLaunch r;
-  r.lines = lines_per_cta(f, staged);
-  r.threads = (r.lines * f.r2 + 31) / 32 * 32;
-  r.smem = static_cast<std::size_t>(r.lines) * (row_line_pitch(f) + (staged ? f.n() + 1 : 0)) * sizeof(float2);
-  r.grid = static_cast<unsigned>((total_lines + r.lines - 1) / r.lines);
-  return r;
-}
-
 // Calls g.template operator()<Max>(factors) when the engine covers length n.
 template <class G>
 bool with_factors(int n, G&& g) {
@@ -556,45 +496,44 @@ bool axis_pass_two(int cols, float2* data, int n_outer, std::size_t so, int n, s
 }
 
 bool rows_r2c_two(const float* x, float2* e, std::size_t rows, int nx, bool clamp, cudaStream_t s) {
-  return with_factors(nx, [&]<int Max>(const Factors& f) {
-    const RowLaunch r = row_launch(f, (rows + 1) / 2, true);
-    const float2* tw = fft_len(nx).tw;
+  return with_factors(nx / 2, [&]<int Max>(const Factors& f) {
+    const RowLaunch r = row_launch(f, rows, true);
     auto kernel = clamp ? k_rows_r2c_two<true, Max> : k_rows_r2c_two<false, Max>;
     ensure_smem(kernel);
-    kernel<<<r.grid, r.threads, r.smem, s>>>(x, e, rows, f, r.lines, tw);
+    kernel<<<r.grid, r.threads, r.smem, s>>>(x, e, rows, f, r.lines, fft_len(nx / 2).tw, fft_len(nx).tw);
     check_launch("rows r2c");
   });
 }
 
 bool rows_c2r_two(const float2* e, float* x, std::size_t rows, int nx, C2rMode mode, float nm2, float inv_k02,
                   cudaStream_t s) {
-  return with_factors(nx, [&]<int Max>(const Factors& f) {
-    const RowLaunch r = row_launch(f, (rows + 1) / 2, false);
-    const float2* tw = fft_len(nx).tw;
+  return with_factors(nx / 2, [&]<int Max>(const Factors& f) {
+    const RowLaunch r = row_launch(f, rows, false);
     auto kernel = mode == C2rMode::index ? k_rows_c2r_two<1, Max> : k_rows_c2r_two<0, Max>;
     ensure_smem(kernel);
-    kernel<<<r.grid, r.threads, r.smem, s>>>(e, x, rows, f, r.lines, tw, nm2, inv_k02);
+    kernel<<<r.grid, r.threads, r.smem, s>>>(e, x, rows, f, r.lines, fft_len(nx / 2).tw, fft_len(nx).tw, nm2, inv_k02);
     check_launch("rows c2r");
   });
 }
 
 bool rows_c2r_r2c_two(float2* e, std::size_t rows, int nx, cudaStream_t s) {
-  return with_factors(nx, [&]<int Max>(const Factors& f) {
-    const RowLaunch r = row_launch(f, (rows + 1) / 2, true);
+  return with_factors(nx / 2, [&]<int Max>(const Factors& f) {
+    const RowLaunch r = row_launch(f, rows, true);
     ensure_smem(k_rows_c2r_r2c_two<Max>);
-    k_rows_c2r_r2c_two<Max><<<r.grid, r.threads, r.smem, s>>>(e, rows, f, r.lines, fft_len(nx).tw);
+    k_rows_c2r_r2c_two<Max><<<r.grid, r.threads, r.smem, s>>>(e, rows, f, r.lines, fft_len(nx / 2).tw, fft_len(nx).tw);
     check_launch("rows c2r r2c");
   });
 }
 
 bool rows_tv_final_r2c_two(const float* b, const float* const p[3], int nz, int ny, int nx, float lambda,
                            float momentum, float* xprev, float2* e, cudaStream_t s) {
-  return with_factors(nx, [&]<int Max>(const Factors& f) {
+  return with_factors(nx / 2, [&]<int Max>(const Factors& f) {
     const std::size_t rows = static_cast<std::size_t>(nz) * ny;
-    const RowLaunch r = row_launch(f, (rows + 1) / 2, true);
+    const RowLaunch r = row_launch(f, rows, true);
     ensure_smem(k_rows_tv_final_r2c_two<Max>);
     k_rows_tv_final_r2c_two<Max><<<r.grid, r.threads, r.smem, s>>>(b, p[0], p[1], p[2], nz, ny, lambda, momentum,
-                                                                   xprev, e, rows, f, r.lines, fft_len(nx).tw);
+                                                                   xprev, e, rows, f, r.lines, fft_len(nx / 2).tw,
+                                                                   fft_len(nx).tw);
     check_launch("rows tv final r2c");
   });
 }

@@ -159,9 +159,9 @@ __device__ __forceinline__ void dft(float2* v) {
 }
 
 // The radices: up to 16 for the first factor, larger ones up to 32 for the second. Kernels are instantiated
-// per class, which sets their registers: radices 2^a 3^b 5^c up to 16, 25 or 32 for the second factor, or
+// per class, which sets their registers: radices 2^a 3^b 5^c up to 16, 24 or 32 for the second factor, or
 // (kAny) all of them, those with factors 7, 11 and 13 too, whose DFTs hold twice the values.
-constexpr int kSmall = 16, kMid = 25, kLarge = 32, kAny = 64;
+constexpr int kSmall = 16, kMid = 24, kLarge = 32, kAny = 64;
 constexpr bool radix(int r) {
   return (r >= 2 && r <= 16) || r == 18 || r == 20 || r == 21 || r == 22 || r == 24 || r == 25 || r == 26 || r == 28 ||
          r == 30 || r == 32;
