@@ -11,8 +11,11 @@
 //   3. rows: m-point inverse FFT along x of the W nonzero columns, then (-1)^(x+y) / N^2
 //      (demodulation), or -- for the Pipeline -- the ratio to the resident background field and its
 //      phase and log-amplitude.
+#include <algorithm>
 #include <cmath>
 
+#include "debug.cuh"
+#include "fft_rows.cuh"
 #include "field.hpp"
 
 namespace qhk {
@@ -158,6 +161,211 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// ---- The same three passes on the two-factor lines (fft_two.cuh), where the lengths have two radices --------
+// Passes 1 and 3 load their rows straight into the first DFT and leave through a natural-order copy in shared
+// memory, one warp per row, so that the window's split and the phase and log-amplitude run once per value on
+// coalesced rows. Pass 2 holds a column's spectrum only inside the crop window. Against the staged passes,
+// 200 x (192^2 -> 96^2): 20, 19 and 25 us from 40, 31 and 33; 49 x (400^2 -> 200^2): 27, 28 and 36 us from 36, 36
+// and 45; 97 x 1024^2 rows 196 us from 318 (the inverse rows of 384 217 from 203).
+
+using twofft::Factors;
+using twofft::RowTile;
+
+constexpr int field_blocks(int max) { return max == twofft::kSmall ? 3 : 2; }
+
+template <int Max>
+__global__ void __launch_bounds__(kThreads, field_blocks(Max))
+    k_holo_rows_two(const float* __restrict__ holo, float2* __restrict__ t1, std::size_t rows, Factors f, int lines,
+                    const float2* __restrict__ tw, const float2* __restrict__ twn, int fx0, int W) {
+  extern __shared__ float2 sm[];
+  const int M = f.n(), N = 2 * M, A = f.r2 | 1, C = twofft::row_line_pitch(f);
+  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + M + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
+  float2* zs = sm + lines * C;
+  const std::size_t row0 = static_cast<std::size_t>(blockIdx.x) * lines;
+  const RowTile r = twofft::row_tile(f, lines);
+  if (r.first) {
+    const bool live = row0 + r.line < rows;
+    twofft::with_first<Max>(f.r1, [&]<int R>() {
+      float2 v[R];
+      const float2* p = reinterpret_cast<const float2*>(holo) + (live ? row0 + r.line : 0) * M + r.j;
+#pragma unroll
+      for (int q = 0; q < R; ++q, p += f.r2) v[q] = live ? *p : make_float2(0.0f, 0.0f);
+      twofft::first_pass<R, true>(v, r.j, tw, sm + r.line * C + r.j, A);
+    });
+  }
+  __syncthreads();
+  if (r.second) {
+    twofft::with_radix<Max>(f.r2, [&]<int R>() {
+      float2 u[R];
+      twofft::second_pass<R, true>(u, sm + r.line2 * C + r.j2 * A, 1);
+#pragma unroll
+      for (int q = 0; q < R; ++q) zs[r.line2 * (M + 1) + r.j2 + f.r1 * q] = u[q];
+    });
+  }
+  __syncthreads();
+  const int warps = static_cast<int>(blockDim.x) >> 5;
+  for (int l = static_cast<int>(threadIdx.x) >> 5; l < lines && row0 + l < rows; l += warps) {
+    const float2* z = zs + l * (M + 1);
+    for (int j = static_cast<int>(threadIdx.x) & 31; j < W; j += 32) {
+      const int fx = fx0 + j;
+      float2 v = make_float2(0.0f, 0.0f);
+      if (fx >= -N / 2 && fx < N / 2) {
+        const int k = fx >= 0 ? fx : -fx;
+        const float2 zk = z[k == M ? 0 : k], zm = z[k == 0 ? 0 : M - k];
+        const float2 ev = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
+        const float2 od = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
+        v = cadd(ev, cmul(__ldg(twn + k), od));
+        if (fx < 0) v.y = -v.y;
+      }
+      t1[(row0 + l) * W + j] = v;
+    }
+  }
+}
+
+// Columns per CTA of pass 2 on the two-factor lines.
+constexpr int kFieldCols = 8;
+
+__host__ __device__ __forceinline__ int field_exchange(const Factors& a, const Factors& b) {
+  const int na = a.r1 * (a.r2 | 1), nb = b.r1 * (b.r2 | 1);
+  return (na > nb ? na : nb) * kFieldCols;
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_holo_cols_two(const float2* __restrict__ t1, float2* __restrict__ t2, Factors fN, Factors fm, int W,
+                    const float2* __restrict__ twN, const float2* __restrict__ twm, int cy, int cx, int dxlo, float r2,
+                    float sign) {
+  extern __shared__ float2 sm[];
+  const int N = fN.n(), m = fm.n();
+  if (!QHK_CHECK(static_cast<std::size_t>(field_exchange(fN, fm) + m * kFieldCols) * sizeof(float2) <=
+                 debug::dynamic_smem_bytes())) {
+    return;
+  }
+  float2* win = sm + field_exchange(fN, fm);  // the crop window's rows, kFieldCols apart
+  const int tid = static_cast<int>(threadIdx.x);
+  const int c = tid % kFieldCols, j = tid / kFieldCols;
+  const int col = static_cast<int>(blockIdx.x) * kFieldCols + c;
+  const bool live = col < W;
+  const std::size_t img = blockIdx.y;
+  const int AN = (fN.r2 | 1) * kFieldCols, Am = (fm.r2 | 1) * kFieldCols;
+  for (int i = tid; i < m * kFieldCols; i += static_cast<int>(blockDim.x)) win[i] = make_float2(0.0f, 0.0f);
+  if (j < fN.r2) {
+    twofft::with_radix<twofft::kAny>(fN.r1, [&]<int R>() {
+      float2 v[R];
+      const float2* p = t1 + (img * N + j) * W + (live ? col : 0);
+#pragma unroll
+      for (int q = 0; q < R; ++q, p += static_cast<std::size_t>(fN.r2) * W) v[q] = live ? *p : make_float2(0.0f, 0.0f);
+      twofft::first_pass<R, true>(v, j, twN, sm + j * kFieldCols + c, AN);
+    });
+  }
+  __syncthreads();
+  if (j < fN.r1) {
+    const int dx = dxlo + col, fx = cx + dx;
+    const bool in_x = live && fx >= -N / 2 && fx < N / 2;
+    twofft::with_radix<twofft::kAny>(fN.r2, [&]<int R>() {
+      float2 u[R];
+      twofft::second_pass<R, true>(u, sm + j * AN + c, kFieldCols);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int k = j + fN.r1 * q;
+        const int fy = k < N / 2 ? k : k - N;
+        const int dy = fy - cy;
+        if (in_x && dy >= -m / 2 && dy < m / 2 && static_cast<float>(dy * dy + dx * dx) <= r2) {
+          win[(m / 2 + dy) * kFieldCols + c] = cscale(u[q], sign);
+        }
+      }
+    });
+  }
+  __syncthreads();
+  if (j < fm.r2) {
+    twofft::with_radix<twofft::kAny>(fm.r1, [&]<int R>() {
+      float2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) v[q] = win[(j + fm.r2 * q) * kFieldCols + c];
+      twofft::first_pass<R, false>(v, j, twm, sm + j * kFieldCols + c, Am);
+    });
+  }
+  __syncthreads();
+  if (j < fm.r1 && live) {
+    twofft::with_radix<twofft::kAny>(fm.r2, [&]<int R>() {
+      float2 u[R];
+      twofft::second_pass<R, false>(u, sm + j * Am + c, kFieldCols);
+      float2* p = t2 + (img * m + j) * W + col;
+#pragma unroll
+      for (int q = 0; q < R; ++q, p += static_cast<std::size_t>(fm.r1) * W) *p = u[q];
+    });
+  }
+}
+
+template <int Mode, int Max>
+__global__ void __launch_bounds__(kThreads, field_blocks(Max))
+    k_field_rows_two(const float2* __restrict__ t2, std::size_t rows, Factors f, int lines, int W, int x0,
+                     const float2* __restrict__ tw, float inv_nn, float2* __restrict__ field,
+                     const float2* __restrict__ bg, float* __restrict__ psi, float* __restrict__ logamp,
+                     std::size_t bg_rows) {
+  extern __shared__ float2 sm[];
+  const int m = f.n(), A = f.r2 | 1, C = twofft::row_line_pitch(f);
+  if (!QHK_CHECK(static_cast<std::size_t>(lines) * (C + m + 1) * sizeof(float2) <= debug::dynamic_smem_bytes())) return;
+  float2* zs = sm + lines * C;
+  const std::size_t row0 = static_cast<std::size_t>(blockIdx.x) * lines;
+  const RowTile r = twofft::row_tile(f, lines);
+  if (r.first) {
+    const bool live = row0 + r.line < rows;
+    const float2* src = t2 + (live ? row0 + r.line : 0) * W;
+    twofft::with_first<Max>(f.r1, [&]<int R>() {
+      float2 v[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int i = r.j + f.r2 * q - x0;
+        v[q] = live && i >= 0 && i < W ? src[i] : make_float2(0.0f, 0.0f);
+      }
+      twofft::first_pass<R, false>(v, r.j, tw, sm + r.line * C + r.j, A);
+    });
+  }
+  __syncthreads();
+  if (r.second) {
+    twofft::with_radix<Max>(f.r2, [&]<int R>() {
+      float2 u[R];
+      twofft::second_pass<R, false>(u, sm + r.line2 * C + r.j2 * A, 1);
+#pragma unroll
+      for (int q = 0; q < R; ++q) zs[r.line2 * (m + 1) + r.j2 + f.r1 * q] = u[q];
+    });
+  }
+  __syncthreads();
+  const int warps = static_cast<int>(blockDim.x) >> 5;
+  for (int l = static_cast<int>(threadIdx.x) >> 5; l < lines && row0 + l < rows; l += warps) {
+    const std::size_t row = row0 + l;
+    const int y = static_cast<int>(row % m);
+    const float2* b_row = Mode == 1 ? bg + (row % bg_rows) * m : nullptr;  // the background stack repeats
+    for (int x = static_cast<int>(threadIdx.x) & 31; x < m; x += 32) {
+      const float2 v = cscale(zs[l * (m + 1) + x], inv_nn * parity(x + y));
+      const std::size_t g = row * m + x;
+      if constexpr (Mode == 0) {
+        field[g] = v;
+      } else {
+        const float2 b = b_row[x];
+        const float d = 1.0f / (b.x * b.x + b.y * b.y);
+        const float re = (v.x * b.x + v.y * b.y) * d;
+        const float im = (v.y * b.x - v.x * b.y) * d;
+        psi[g] = atan2f(im, re);
+        logamp[g] = logf(hypotf(re, im));
+      }
+    }
+  }
+}
+
+// Any two radices for a column of pass 2 (both factors up to 32, so that 1024 = 32 x 32 has them too), the
+// larger one second.
+bool column_factors(int n, Factors* f) {
+  for (int r1 = 32; r1 >= 2; --r1) {
+    const int r2 = n / r1;
+    if (r1 * r2 == n && r2 >= r1 && twofft::radix(r1) && twofft::radix(r2)) {
+      *f = Factors{r1, r2};
+      return true;
+    }
+  }
+  return false;
+}
+
 int rows_per_cta(int len) {
   int c = 16;
   while (c > 1 && 2 * static_cast<std::size_t>(len + 1) * (c + 1) * sizeof(float2) > 64 * 1024) c /= 2;
@@ -209,7 +417,16 @@ void FieldPlan::spectra(const float* holo, int first, int valid, cudaStream_t s)
   const FftLen& Lo = fft_len(m);
   const std::size_t rows = static_cast<std::size_t>(valid) * N;
   float2* t1 = t1_.get() + static_cast<std::size_t>(first) * N * W_;
-  {
+  Factors f;
+  if (fft_reg_engine_enabled() && twofft::factors(N / 2, &f)) {
+    const twofft::RowLaunch r = twofft::row_launch(f, rows, true);
+    twofft::with_class(f, [&]<int Max>() {
+      ensure_smem(k_holo_rows_two<Max>);
+      k_holo_rows_two<Max><<<r.grid, r.threads, r.smem, s>>>(holo, t1, rows, f, r.lines, Lm.tw, Ln.tw,
+                                                            plan_.cx + dxlo_, W_);
+    });
+    check_launch("field rows");
+  } else {
     const int c = rows_per_cta(N / 2);
     const std::size_t smem = 2 * static_cast<std::size_t>(N / 2 + 1) * (c + 1) * sizeof(float2);
     const unsigned grid = static_cast<unsigned>((rows + c - 1) / c);
@@ -229,7 +446,15 @@ void FieldPlan::spectra(const float* holo, int first, int valid, cudaStream_t s)
 #undef QHK_ROWS
     check_launch("field rows");
   }
-  {
+  Factors fN, fm;
+  if (fft_reg_engine_enabled() && column_factors(N, &fN) && column_factors(m, &fm)) {
+    const std::size_t smem = static_cast<std::size_t>(field_exchange(fN, fm) + m * kFieldCols) * sizeof(float2);
+    ensure_smem(k_holo_cols_two);
+    k_holo_cols_two<<<dim3((W_ + kFieldCols - 1) / kFieldCols, valid), kFieldCols * std::max(fN.r2, fm.r2), smem, s>>>(
+        t1, t2_.get() + static_cast<std::size_t>(first) * m * W_, fN, fm, W_, Ln.tw, Lo.tw, plan_.cy, plan_.cx, dxlo_, r2_,
+        parity(plan_.cy + plan_.cx));
+    check_launch("field columns");
+  } else {
     const int big = std::max(N, m);
     int c = 16;
     while (c > 1 && 2 * static_cast<std::size_t>(big) * c * sizeof(float2) > 72 * 1024) c /= 2;
@@ -261,11 +486,23 @@ void FieldPlan::finish(int mode, float2* field, const float2* bg, float* psi, fl
   const FftLen& Lo = fft_len(m);
   require(images >= 0 && images <= count_, "fields: image count beyond the plan");
   const std::size_t rows = static_cast<std::size_t>(images > 0 ? images : count_) * m;
+  const int x0 = m / 2 + dxlo_;
+  const float inv_nn = 1.0f / static_cast<float>(static_cast<std::size_t>(N) * N);
+  Factors f;
+  if (fft_reg_engine_enabled() && twofft::factors(m, &f)) {
+    const twofft::RowLaunch r = twofft::row_launch(f, rows, true);
+    twofft::with_class(f, [&]<int Max>() {
+      auto kernel = mode == 0 ? k_field_rows_two<0, Max> : k_field_rows_two<1, Max>;
+      ensure_smem(kernel);
+      kernel<<<r.grid, r.threads, r.smem, s>>>(t2_.get(), rows, f, r.lines, W_, x0, Lo.tw, inv_nn, field, bg, psi,
+                                               logamp, bg_rows);
+    });
+    check_launch("field inverse rows");
+    return;
+  }
   const int c = rows_per_cta(m);
   const std::size_t smem = 2 * static_cast<std::size_t>(m) * (c + 1) * sizeof(float2);
   const unsigned grid = static_cast<unsigned>((rows + c - 1) / c);
-  const int x0 = m / 2 + dxlo_;
-  const float inv_nn = 1.0f / static_cast<float>(static_cast<std::size_t>(N) * N);
 #define QHK_FIN(C)                                                                                        \
   case C:                                                                                                 \
     if (mode == 0) {                                                                                      \
