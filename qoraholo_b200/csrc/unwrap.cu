@@ -597,8 +597,9 @@ int unwrap_line_threads(int n) {
 // inputs (q, r2 - q) for pairs of outputs (m, r2 - m), r2^2 multiplications, four output pairs per thread
 // against shared roots. A tile has `lines` lines, the fastest index of every shared array, so that no
 // access has bank conflicts and no index needs a division. What bounds the passes is the latency of their
-// phases; 200 images of sides 96 .. 640 in steps of 8 (18 M pixels): the three passes take 0.96 ms, on the
-// staged engine 9.5 ms; one image of 120 x 160: 24 us from 40.
+// phases: 16 lines per tile up to a side of 320, 8 beyond, and in a stack kernels of the factors' class only.
+// 200 images of sides 96 .. 640 in steps of 8 (18 M pixels): the three passes take 0.9 ms, on the staged engine
+// 9.5 ms; 49 images of 200^2 26, 30 and 28 us from 33, 46 and 37; one of 120 x 160 27 us from 40.
 struct DctLine {
   int n = 0;  // side; 0: not on this engine
   int r1 = 0, r2 = 0;
@@ -641,12 +642,12 @@ DctLine dct_line(int n) {
     l.direct = 1;
   }
   l.n = n;
-  l.lines = n < 128 ? 16 : 8;
+  l.lines = n <= 320 ? 16 : 8;
   return l;
 }
 
 // First pass of the tile: load(line, m) gives input m of a line; slots (k1, j) of xs.
-template <bool Fwd, class Load>
+template <bool Fwd, int Max, class Load>
 __device__ __forceinline__ void dct_first(const DctLine& f, float2* xs, const float2* __restrict__ twn, Load load) {
   const int P = f.r2 | 1;
   const auto run = [&]<int R>() {
@@ -668,16 +669,16 @@ __device__ __forceinline__ void dct_first(const DctLine& f, float2* xs, const fl
   if (f.r1 == 1) {
     run.template operator()<1>();
   } else {
-    twofft::with_first<twofft::kAny>(f.r1, run);
+    twofft::with_first<Max>(f.r1, run);
   }
 }
 
 // Second pass: sink(line, k, value) receives output k of a line.
-template <bool Fwd, class Sink>
+template <bool Fwd, int Max, class Sink>
 __device__ __forceinline__ void dct_second(const DctLine& f, const float2* xs, const float2* roots, Sink sink) {
   const int P = f.r2 | 1, log = f.log_lines();
   if (!f.direct) {
-    twofft::with_radix<twofft::kAny>(f.r2, [&]<int R>() {
+    twofft::with_radix<Max>(f.r2, [&]<int R>() {
       for (int i = static_cast<int>(threadIdx.x); i < (f.r1 << log); i += kThreads) {
         const int line = i & (f.lines - 1), k1 = i >> log;
         float2 u[R];
@@ -740,6 +741,7 @@ __device__ __forceinline__ void load_roots(const DctLine& f, float2* roots, cons
 }
 
 // Pass 1 on rows y0 .. y0 + lines - 1.
+template <int Max>
 __device__ __forceinline__ void div_dctx_tile_two(const float* __restrict__ psi, float* __restrict__ d1, int ny,
                                                   const DctLine& f, const float2* __restrict__ twn,
                                                   const float2* __restrict__ dtw, int y0, float2* sm) {
@@ -777,9 +779,9 @@ __device__ __forceinline__ void div_dctx_tile_two(const float* __restrict__ psi,
     zs[i] = make_float2(r[0], r[1]);
   }
   __syncthreads();
-  dct_first<true>(f, xs, twn, [&](int line, int m) { return zs[(m << log) + line]; });
+  dct_first<true, Max>(f, xs, twn, [&](int line, int m) { return zs[(m << log) + line]; });
   __syncthreads();
-  dct_second<true>(f, xs, roots, [&](int line, int k, float2 v) { zs[(k << log) + line] = v; });
+  dct_second<true, Max>(f, xs, roots, [&](int line, int k, float2 v) { zs[(k << log) + line] = v; });
   __syncthreads();
   for (int i = static_cast<int>(threadIdx.x); i < ((h + 1) << log); i += kThreads) {
     const int row = i & (f.lines - 1), k = i >> log;
@@ -795,6 +797,7 @@ __device__ __forceinline__ void div_dctx_tile_two(const float* __restrict__ psi,
 }
 
 // Pass 2 on columns c0 .. c0 + lines - 1 of an image of height f.n.
+template <int Max>
 __device__ __forceinline__ void dcty_solve_tile_two(const float* __restrict__ d1, float* __restrict__ d2, int nx,
                                                     const DctLine& f, const float2* __restrict__ twn,
                                                     const float2* __restrict__ dtw, const float* __restrict__ cos_y,
@@ -805,14 +808,14 @@ __device__ __forceinline__ void dcty_solve_tile_two(const float* __restrict__ d1
   float2* zs = xs + f.area();
   float2* roots = zs + f.area();
   load_roots(f, roots, twn);
-  dct_first<true>(f, xs, twn, [&](int line, int m) {
+  dct_first<true, Max>(f, xs, twn, [&](int line, int m) {
     const float* in = d1 + c0 + line;
     return c0 + line < nx ? make_float2(in[static_cast<std::size_t>(makhoul_x(2 * m, n)) * nx],
                                         in[static_cast<std::size_t>(makhoul_x(2 * m + 1, n)) * nx])
                           : make_float2(0.0f, 0.0f);
   });
   __syncthreads();
-  dct_second<true>(f, xs, roots, [&](int line, int k, float2 v) { zs[(k << log) + line] = v; });
+  dct_second<true, Max>(f, xs, roots, [&](int line, int k, float2 v) { zs[(k << log) + line] = v; });
   __syncthreads();
   for (int i = static_cast<int>(threadIdx.x); i < ((h + 1) << log); i += kThreads) {
     const int line = i & (f.lines - 1), k = i >> log, col = c0 + line;
@@ -827,12 +830,12 @@ __device__ __forceinline__ void dcty_solve_tile_two(const float* __restrict__ d1
     xs[i] = cmulc(make_float2(ak, k == 0 ? 0.0f : -ank), __ldg(dtw + k));  // A[k]
   }
   __syncthreads();
-  dct_first<false>(f, zs, twn, [&](int line, int k) {
+  dct_first<false, Max>(f, zs, twn, [&](int line, int k) {
     return idct_merge(xs[(k << log) + line], xs[((h - k) << log) + line], k, twn);
   });
   __syncthreads();
   const float inv = 1.0f / static_cast<float>(n);
-  dct_second<false>(f, zs, roots, [&](int line, int m, float2 v) {
+  dct_second<false, Max>(f, zs, roots, [&](int line, int m, float2 v) {
     if (c0 + line >= nx) return;
     float* out = d2 + c0 + line;
     out[static_cast<std::size_t>(makhoul_x(2 * m, n)) * nx] = v.x * inv;
@@ -841,6 +844,7 @@ __device__ __forceinline__ void dcty_solve_tile_two(const float* __restrict__ d1
 }
 
 // Pass 3 on rows y0 .. y0 + lines - 1, in place, with the congruence partial sums (idctx_tile).
+template <int Max>
 __device__ __forceinline__ void idctx_tile_two(float* __restrict__ phi, const float* __restrict__ psi, int ny,
                                                const DctLine& f, const float2* __restrict__ twn,
                                                const float2* __restrict__ dtw, int y0, double* __restrict__ pair,
@@ -866,10 +870,10 @@ __device__ __forceinline__ void idctx_tile_two(float* __restrict__ phi, const fl
     zs[i] = idct_merge(ak, am, k, twn);
   }
   __syncthreads();
-  dct_first<false>(f, xs, twn, [&](int line, int k) { return zs[(k << log) + line]; });
+  dct_first<false, Max>(f, xs, twn, [&](int line, int k) { return zs[(k << log) + line]; });
   __syncthreads();
   const float inv = 1.0f / static_cast<float>(n);
-  dct_second<false>(f, xs, roots, [&](int line, int m, float2 v) {
+  dct_second<false, Max>(f, xs, roots, [&](int line, int m, float2 v) {
     F[line * pn + makhoul_x(2 * m, n)] = v.x * inv;
     F[line * pn + makhoul_x(2 * m + 1, n)] = v.y * inv;
   });
@@ -902,31 +906,45 @@ __device__ __forceinline__ void idctx_tile_two(float* __restrict__ phi, const fl
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
+template <int Max>
+__global__ void __launch_bounds__(kThreads, Max == twofft::kSmall ? 3 : 2)
     k_div_dctx_two(const float* __restrict__ psi, float* __restrict__ d1, int ny, DctLine f,
                    const float2* __restrict__ twn, const float2* __restrict__ dtw) {
   extern __shared__ __align__(16) float2 sm[];
   const std::size_t img = static_cast<std::size_t>(blockIdx.y) * ny * f.n;
-  div_dctx_tile_two(psi + img, d1 + img, ny, f, twn, dtw, static_cast<int>(blockIdx.x) * f.lines, sm);
+  div_dctx_tile_two<Max>(psi + img, d1 + img, ny, f, twn, dtw, static_cast<int>(blockIdx.x) * f.lines, sm);
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
+template <int Max>
+__global__ void __launch_bounds__(kThreads, Max == twofft::kSmall ? 3 : 2)
     k_dcty_solve_two(const float* __restrict__ d1, float* __restrict__ d2, int nx, DctLine f,
                      const float2* __restrict__ twn, const float2* __restrict__ dtw,
                      const float* __restrict__ cos_y, const float* __restrict__ cos_x) {
   extern __shared__ __align__(16) float2 sm[];
   const std::size_t img = static_cast<std::size_t>(blockIdx.y) * f.n * nx;
-  dcty_solve_tile_two(d1 + img, d2 + img, nx, f, twn, dtw, cos_y, cos_x, static_cast<int>(blockIdx.x) * f.lines, sm);
+  dcty_solve_tile_two<Max>(d1 + img, d2 + img, nx, f, twn, dtw, cos_y, cos_x, static_cast<int>(blockIdx.x) * f.lines, sm);
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
+template <int Max>
+__global__ void __launch_bounds__(kThreads, Max == twofft::kSmall ? 3 : 2)
     k_idctx_two(float* __restrict__ phi, const float* __restrict__ psi, int ny, DctLine f,
                 const float2* __restrict__ twn, const float2* __restrict__ dtw, double* __restrict__ partial) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ double red[2][kThreads];
   const std::size_t img = static_cast<std::size_t>(blockIdx.y) * ny * f.n;
-  idctx_tile_two(phi + img, psi + img, ny, f, twn, dtw, static_cast<int>(blockIdx.x) * f.lines,
+  idctx_tile_two<Max>(phi + img, psi + img, ny, f, twn, dtw, static_cast<int>(blockIdx.x) * f.lines,
                  partial + (static_cast<std::size_t>(blockIdx.y) * gridDim.x + blockIdx.x) * 2, sm, red);
+}
+
+// Calls g.template operator()<Max>() with the kernel class of the line's factors (fft_two.cuh), of which a stack
+// needs one; a batch of uneven images takes kAny.
+template <class G>
+void with_line_class(const DctLine& f, G&& g) {
+  if (f.direct) {
+    g.template operator()<twofft::kAny>();
+  } else {
+    twofft::with_class(twofft::Factors{f.r1, f.r2}, g);
+  }
 }
 
 // The three passes of a stack on this engine; false when it does not run lines of that length.
@@ -934,8 +952,10 @@ bool pass1_two(const float* psi, float* d1, int count, int ny, int nx, const flo
                cudaStream_t s) {
   const DctLine f = dct_line(nx);
   if (f.n == 0) return false;
-  ensure_smem(k_div_dctx_two);
-  k_div_dctx_two<<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(psi, d1, ny, f, twn, dtw);
+  with_line_class(f, [&]<int Max>() {
+    ensure_smem(k_div_dctx_two<Max>);
+    k_div_dctx_two<Max><<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(psi, d1, ny, f, twn, dtw);
+  });
   check_launch("unwrap pass 1");
   return true;
 }
@@ -943,9 +963,11 @@ bool pass2_two(const float* d1, float* phi, int count, int ny, int nx, const flo
                const float* cos_y, const float* cos_x, cudaStream_t s) {
   const DctLine f = dct_line(ny);
   if (f.n == 0) return false;
-  ensure_smem(k_dcty_solve_two);
-  k_dcty_solve_two<<<dim3((nx + f.lines - 1) / f.lines, count), kThreads, f.cols_smem(), s>>>(d1, phi, nx, f, twn, dtw,
-                                                                                              cos_y, cos_x);
+  with_line_class(f, [&]<int Max>() {
+    ensure_smem(k_dcty_solve_two<Max>);
+    k_dcty_solve_two<Max><<<dim3((nx + f.lines - 1) / f.lines, count), kThreads, f.cols_smem(), s>>>(d1, phi, nx, f, twn, dtw,
+                                                                                                cos_y, cos_x);
+  });
   check_launch("unwrap pass 2");
   return true;
 }
@@ -953,9 +975,11 @@ bool pass3_two(float* phi, const float* psi, int count, int ny, int nx, const fl
                double* partial, cudaStream_t s) {
   const DctLine f = dct_line(nx);
   if (f.n == 0) return false;
-  ensure_smem(k_idctx_two);
-  k_idctx_two<<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(phi, psi, ny, f, twn, dtw,
-                                                                                         partial);
+  with_line_class(f, [&]<int Max>() {
+    ensure_smem(k_idctx_two<Max>);
+    k_idctx_two<Max><<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(phi, psi, ny, f, twn, dtw,
+                                                                                           partial);
+  });
   check_launch("unwrap pass 3");
   return true;
 }
@@ -1329,7 +1353,7 @@ __global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.nx, QHK_R1)
     } else if constexpr (Kind == kTwo) {
-      div_dctx_tile_two(psi + im.offset, d1 + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, sm);
+      div_dctx_tile_two<twofft::kAny>(psi + im.offset, d1 + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, sm);
     } else {
       QHK_ROWS_SWITCH(im.rows, QHK_P1)
     }
@@ -1356,7 +1380,7 @@ __global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.ny, QHK_R2)
     } else if constexpr (Kind == kTwo) {
-      dcty_solve_tile_two(d1 + im.offset, phi + im.offset, im.nx, im.line_y, im.Ly.tw, im.dtw_y, im.cos_y, im.cos_x,
+      dcty_solve_tile_two<twofft::kAny>(d1 + im.offset, phi + im.offset, im.nx, im.line_y, im.Ly.tw, im.dtw_y, im.cos_y, im.cos_x,
                           w.y * im.line_y.lines, sm);
     } else {
       QHK_ROWS_SWITCH(im.cols, QHK_P2)
@@ -1385,7 +1409,7 @@ __global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.nx, QHK_R3)
     } else if constexpr (Kind == kTwo) {
-      idctx_tile_two(phi + im.offset, psi + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, pair,
+      idctx_tile_two<twofft::kAny>(phi + im.offset, psi + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, pair,
                      sm, red);
     } else {
       QHK_ROWS_SWITCH(im.rows, QHK_P3)
