@@ -1217,15 +1217,19 @@ std::size_t fgp_smem(int nx, int ty) {
 // where the caller has the fourth dual triplet); the default is the tallest of at most 4 rows of
 // the one-step form within 110 KiB.
 template <int VEC>
-std::vector<int> fgp_rows_candidates(int nx, bool two_step) {
+std::vector<int> fgp_rows_candidates(int ny, int nx, bool two_step) {
   std::vector<int> out;
   const int tx = nx / VEC;
   if (VEC == 4 && two_step) {
     for (const int ty : {8, 4, 2})
       if (fgp2_fits(nx, ty)) out.push_back(2 * kFgpVariantScale + ty);
-    for (int t = 1; t <= kMaxWindows; ++t) {
+    // Windows within a tenth of the fewest tiles, so that plans time one or two of them.
+    const Fgp2Window fewest = fgp2_fewest_tiles(ny, nx);
+    const auto tiles = [&](const Fgp2Window& w) { return w.xtiles * ((ny + w.ty - 1) / w.ty); };
+    for (int t = 1; t <= kMaxWindows && fewest.ty > 0; ++t) {
       const Fgp2Window w = fgp2_window(nx, t);
-      if (w.ty > (t == 1 ? 8 : 7)) out.push_back(3 * kFgpVariantScale + t);
+      if (w.ty == 0 || (t == 1 && w.ty == 8) || 10 * tiles(w) > 11 * tiles(fewest)) continue;
+      out.push_back(3 * kFgpVariantScale + t);
     }
   }
   for (const int variant : {1, 0}) {
@@ -1668,7 +1672,7 @@ void tune_fgp_rows(float* b, TvBuffers& t, int nz, int ny, int nx, float lambda,
       w.rout[c] = t.v[3][c];
     }
   }
-  autotune(fgp_key<VEC>(nz, ny, nx), fgp_rows_candidates<VEC>(nx, t.has_fourth()), fgp_rows_default<VEC>(nx),
+  autotune(fgp_key<VEC>(nz, ny, nx), fgp_rows_candidates<VEC>(ny, nx, t.has_fourth()), fgp_rows_default<VEC>(nx),
            [&](int choice) {
              const FgpShape sh = fgp_shape_rows<VEC>(nz, ny, nx, choice);
              if (sh.two_step()) {
