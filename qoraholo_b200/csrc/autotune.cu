@@ -125,7 +125,6 @@ int autotune(const TuneKey& key, const std::vector<int>& candidates, int fallbac
   }
   for (int turn = 0; turn < kTurns; ++turn) {
     for (auto& [c, us] : e.timings) {
-      run(c);
       start.record(s);
       for (int r = 0; r < each; ++r) run(c);
       stop.record(s);

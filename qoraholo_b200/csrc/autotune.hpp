@@ -2,7 +2,7 @@
 // fastest per (device, family, shape), for the rest of the process.
 //
 // Tuning runs when a plan is built (never inside a stream capture): each candidate is launched on
-// the plan's own scratch buffers, twice to warm up and then `reps` times between CUDA events, and
+// the plan's own scratch buffers, once to warm up and then in turns, `reps` times in all, between CUDA events, and
 // the candidate with the smallest time wins. Kernels then read their shape from the table, falling
 // back to a fixed heuristic when a shape was never tuned (or tuning is off: QHK_AUTOTUNE=0). With
 // QHK_AUTOTUNE_FILE set, choices are also read from and appended to that file, so that another run

@@ -36,3 +36,23 @@ def test_slice_passes_match_the_oracle(cuda, n, count):
     assert rel_err(y.detach().cpu().numpy(), want) < 1e-5
     assert rel_err(grads[0], want_grad) < 2e-5
     assert np.array_equal(grads[0], grads[1])
+
+
+def test_passes_over_the_views_agree_with_one_pass(cuda):
+    """Enough views that the plan takes them in several passes: fields bitwise those of one pass, the gradient
+    up to the order in which the passes' sums are added (two passes of float32 sums: 4e-7)."""
+    from oracle import qh_oracle as O
+    from qoraholo_b200.autograd import BpmModel
+
+    n, nz, count = 256, 3, 40  # 73 MB of state
+    rng = np.random.default_rng(3)
+    il = O.circular_scan(count, 0.9, G)
+    ri = cuda.from_numpy((G[1] + 0.03 * rng.random((nz, n, n))).astype(np.float32)).cuda()
+    out = []
+    for chunk in (0, count):
+        x = ri.clone().requires_grad_(True)
+        y = BpmModel(nz, n, il, G, checkpoint_every=2, chunk=chunk)(x)
+        y.backward(y.detach() - 1)
+        out.append((y.detach().cpu().numpy(), x.grad.cpu().numpy()))
+    assert np.array_equal(out[0][0], out[1][0])
+    assert rel_err(out[0][1], out[1][1]) < 4e-7
