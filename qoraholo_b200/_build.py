@@ -31,7 +31,10 @@ BUILD = PKG / "_build"
 INCLUDE = ROOT / "include"
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-std=c++20", "-O3", "--split-compile=0", *ARCH, "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler",
+# Each unit is optimised as a whole. With --split-compile the register allocation of nearly every kernel changes:
+# the one-step TV kernels were cut from 80-126 registers to 38-56 and two GP passes and the BPM row pass spilled
+# (prox of 100 x 200 x 150 0.75 ms without it, 1.07 ms with it; FISTA-TV of 256^3 22.4 and 23.6 ms).
+NVCC_FLAGS = ["-std=c++20", "-O3", *ARCH, "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler",
               "-fPIC,-ffp-contract=off", f"-I{INCLUDE}", f"-I{CSRC}"]
 CXX_FLAGS = ["-std=c++20", "-O2", "-fPIC", "-ffp-contract=off", f"-I{INCLUDE}", f"-I{CSRC}"]
 
@@ -49,11 +52,18 @@ def _headers():
     return list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.hpp")) + list(INCLUDE.rglob("*.h*"))
 
 
-def _stale(obj: Path, src: Path) -> bool:
-    """True when obj must be rebuilt: it or its dependency list (obj.d, written by the compiler's -MD
-    -MF) is missing, or the source or any header it included is newer."""
-    dep = obj.with_suffix(".d")
-    if not obj.exists() or not dep.exists():
+def _command_record(obj: Path) -> Path:
+    return obj.with_suffix(".cmd")
+
+
+def _stale(obj: Path, src: Path, cmd) -> bool:
+    """True when obj must be rebuilt by `cmd`: it, its dependency list (obj.d, written by the compiler's -MD
+    -MF) or the record of its command (obj.cmd) is missing, it was compiled by another command, or the source
+    or any header it included is newer."""
+    dep, record = obj.with_suffix(".d"), _command_record(obj)
+    if not obj.exists() or not dep.exists() or not record.exists():
+        return True
+    if record.read_text() != _command_text(cmd):
         return True
     text = dep.read_text().replace("\\\n", " ")
     files = [Path(t) for t in text.partition(":")[2].split()]
@@ -68,12 +78,18 @@ def _run(cmd):
     return r
 
 
+def _command_text(cmd) -> str:
+    return "\n".join(map(str, cmd)) + "\n"
+
+
 def _compile(cmd):
-    """One compile job; an object whose source or headers changed while it compiled is dated back to the
-    start of the compile, so that the next build compiles it again."""
+    """One compile job, its command recorded beside the object; an object whose source or headers changed while
+    it compiled is dated back to the start of the compile, so that the next build compiles it again."""
     t0 = time.time()
-    _run(cmd)
     obj = Path(cmd[cmd.index("-o") + 1])
+    _command_record(obj).unlink(missing_ok=True)  # a failed compile leaves the earlier object without a record
+    _run(cmd)
+    _command_record(obj).write_text(_command_text(cmd))
     dep = obj.with_suffix(".d")
     if dep.exists():
         files = [Path(t) for t in dep.read_text().replace("\\\n", " ").partition(":")[2].split()]
@@ -93,8 +109,9 @@ def build_qhk(force=False) -> Path:
     for src in sources:
         obj = BUILD / (src.stem + ".o")
         objs.append(obj)
-        if force or _stale(obj, src):
-            jobs.append([NVCC, *NVCC_FLAGS, "-MD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)])
+        cmd = [NVCC, *NVCC_FLAGS, "-MD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)]
+        if force or _stale(obj, src, cmd):
+            jobs.append(cmd)
     _compile_many(jobs)
     if force or jobs or not LIB_QHK.exists() or LIB_QHK.stat().st_mtime < _newest(objs):
         _run([NVCC, *ARCH, "-shared", "-o", str(LIB_QHK), *map(str, objs)])
@@ -118,9 +135,10 @@ def build_qhk_debug(force=False) -> Path:
         obj = BUILD / (src.stem + ".o")
         if _uses_debug_checks(obj):
             obj = BUILD_DEBUG / (src.stem + ".o")
-            if force or _stale(obj, src):
-                jobs.append([NVCC, *NVCC_FLAGS, "-DQHK_DEBUG", "-MD", "-MF", str(obj.with_suffix(".d")), "-c",
-                             str(src), "-o", str(obj)])
+            cmd = [NVCC, *NVCC_FLAGS, "-DQHK_DEBUG", "-MD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o",
+                   str(obj)]
+            if force or _stale(obj, src, cmd):
+                jobs.append(cmd)
         objs.append(obj)
     _compile_many(jobs)
     if force or jobs or not LIB_QHK_DEBUG.exists() or LIB_QHK_DEBUG.stat().st_mtime < _newest(objs):
@@ -138,8 +156,9 @@ def build_host(force=False) -> Path | None:
     for src in sources:
         obj = BUILD / ("host_" + src.stem + ".o")
         objs.append(obj)
-        if force or _stale(obj, src):
-            jobs.append(["g++", *CXX_FLAGS, "-MD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)])
+        cmd = ["g++", *CXX_FLAGS, "-MD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)]
+        if force or _stale(obj, src, cmd):
+            jobs.append(cmd)
     _compile_many(jobs)
     if force or jobs or not LIB_HOST.exists() or LIB_HOST.stat().st_mtime < max(_newest(objs), LIB_QHK.stat().st_mtime):
         _run(["g++", "-shared", "-o", str(LIB_HOST), *map(str, objs), f"-L{PKG}", "-lqhk", "-Wl,-rpath,$ORIGIN"])
