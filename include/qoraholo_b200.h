@@ -435,8 +435,9 @@ int qhk_bpm_vjp(const float* x, int nz, int n, const void* r, const float* illum
  * reference's CUDA backend (src/cuda/bpm.cu:126-199; forward and adjoint sweeps, envelopes stored
  * for every slice) with a plan that keeps, per illumination, only the spectrum entering every
  * `checkpoint_every`-th slice (0: every envelope, as the reference) and recomputes each segment of
- * slices before sweeping it backwards. `chunk` illuminations run per device pass (0: all, or, where their state exceeds half of L2 and slices are
- * checkpointed, equal passes that stay within it). */
+ * slices before sweeping it backwards. `chunk` illuminations run per device pass (0: all, or, where
+ * slices are checkpointed and two passes keep in L2 what one does not, half of them; the fields are the
+ * same, the gradient differs by the order of the passes' sums). */
 typedef struct qhk_bpm_plan qhk_bpm_plan;
 int qhk_bpm_plan_create(qhk_bpm_plan** plan, int nz, int n, const float* illum_fyfx, int count,
                         const qhk_geometry* geometry, int obliquity, int chunk, int checkpoint_every);

@@ -120,7 +120,8 @@ class BpmModel(torch.nn.Module):
 
     Same model and geometry conventions as ``qoraholo_b200.bpm_forward`` (dz = pixel, the volume
     centred on z = 0 of the detection plane, ``obliquity`` weighting). ``checkpoint_every`` slices per
-    stored spectrum; ``chunk`` illuminations per device pass (0: all, in equal passes within half of L2)."""
+    stored spectrum; ``chunk`` illuminations per device pass (0: all, or half of
+    them where that keeps a pass's state in L2)."""
 
     def __init__(self, nz, n, illuminations, geometry, obliquity=True, checkpoint_every=16, chunk=0):
         super().__init__()

@@ -748,6 +748,7 @@ void with_slice_shape(int n, Reg&& reg, Two&& two) {
 
 // Views per group of the row passes (the groups the gradient is summed in).
 int slice_views(int n) { return n == 64 || n == 128 ? regfft::RowTile<8>::R : n == 256 ? regfft::RowTile<16>::R : kSliceViews; }
+int slice_groups(int n, int views) { return (views + slice_views(n) - 1) / slice_views(n); }
 
 void slice_cols(int n, int mode, const ColArgs& a, int nb, cudaStream_t s) {
   with_slice_shape(
@@ -772,7 +773,7 @@ void slice_gradient(int n, bool forward, float2* data, const float2* env, const 
   if (grad) {
     const std::size_t plane = static_cast<std::size_t>(n) * n;
     k_gradient_groups<<<static_cast<unsigned>((plane + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        part, (nb + slice_views(n) - 1) / slice_views(n), plane, gscale, phase, grad);
+        part, slice_groups(n, nb), plane, gscale, phase, grad);
     check_launch("bpm gradient groups");
   }
 }
@@ -963,6 +964,22 @@ BpmTablesHost bpm_tables(int n, int nz, const float* il, int count, float wavele
   return t;
 }
 
+// Two equal passes where one pass's state (spectrum, envelope, propagator and obliquity, 28 bytes per pixel and
+// view, touched by every slice) is more than L2 keeps from slice to slice and half of it is not, and the halves make
+// no more groups of views than the whole. One pass against two, gradients of 16 to 128 slices: 256^2 with 49 views 24.9 and 22.8 ms,
+// with 64 views 16.7 and 16.1; 264^2 and 384^2 with 49 and 20 views 12.3 and 10.0, 7.6 and 6.5; forty sides and counts
+// in this range 1.00 to 1.22 times. Outside it one pass: with another group (256^2, 40 views: 20.1 and 21.6 ms),
+// below 72 MB (352^2, 20 views: 6.0 and 6.6), above 112 MB (480^2, 20 views: 10.4 and 10.8; 512^2, 49 views, nine
+// passes: 17.1 and 20.5), and for sides up to 240, where either can be faster (200^2, 64 views: 8.8 and 7.7; 224^2,
+// 49 views: 6.0 and 6.7).
+int bpm_default_chunk(int n, int count) {
+  constexpr std::size_t kViewBytes = 28, kLow = std::size_t{72} << 20, kHigh = std::size_t{112} << 20;
+  const std::size_t state = kViewBytes * n * n * count;
+  if (n <= 240 || !slice_covers(n) || state < kLow || state > kHigh) return count;
+  const int half = (count + 1) / 2;
+  return slice_groups(n, half) + slice_groups(n, count - half) > slice_groups(n, count) ? count : half;
+}
+
 BpmPlan::BpmPlan(const BpmTablesHost& t, int chunk, bool store, int checkpoint_every)
     : t_(t), chunk_(chunk), store_on_(store && checkpoint_every <= 0), every_(std::max(checkpoint_every, 0)) {
   require(t.n >= 4 && t.n % 2 == 0 && t.nz >= 1 && t.count >= 1, "bpm: invalid tables");
@@ -1136,7 +1153,7 @@ void BpmPlan::adjoint(const float* x, const float2* residual_or_null, int first,
   // Two passes per slice on the two-factor engine: k_slice_gradient (inverse rows, gradient, conj(screen),
   // forward rows) and k_slice_cols<kSplitInv> (forward columns, split, inverse columns).
   if (slice_covers(t_.n)) {
-    const int groups = (nb + slice_views(t_.n) - 1) / slice_views(t_.n);
+    const int groups = slice_groups(t_.n, nb);
     const auto split = [&](const float2* coef, int has_back, float* slice_grad) {
       ColArgs c{};
       c.data = w_.get();

@@ -22,6 +22,9 @@ struct BpmTablesHost {
 BpmTablesHost bpm_tables(int n, int nz, const float* illum_fyfx, int count, float wavelength, float n_medium,
                          float na, float pixel, bool obliquity);
 
+// Illuminations per device pass of a checkpointed plan whose caller names none: all, or half of them.
+int bpm_default_chunk(int n, int count);
+
 class BpmPlan {
  public:
   // chunk: illuminations per device pass; store: keep the envelope in front of every screen for

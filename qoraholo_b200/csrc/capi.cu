@@ -705,14 +705,10 @@ int qhk_bpm_plan_create(qhk_bpm_plan** plan, int nz, int n, const float* illum_f
     auto p = std::make_unique<qhk_bpm_plan>();
     p->tables = checked_tables(nz, n, count, illum_fyfx, geometry, obliquity != 0);
     p->n_medium = geometry->n_medium;
-    // By default all illuminations, in equal passes whose state (spectrum, envelope, propagator and obliquity, 28
-    // bytes per pixel and view) stays within half of L2 from slice to slice: 256^2 x 128, 49 views as 25 + 24 take
-    // 21.9-22.3 ms per gradient, in one pass 22.2-25.3 from one allocation to the next. (160^2, 24 views fit: one
-    // pass 3.9 ms, two 7.1.) Without checkpoints one pass holds every envelope.
-    constexpr std::size_t kViewBytes = 28, kResident = std::size_t{64} << 20;
-    const std::size_t state = kViewBytes * n * n * count;
-    const int passes = checkpoint_every > 0 ? static_cast<int>((state + kResident - 1) / kResident) : 1;
-    p->chunk = chunk > 0 ? std::min(chunk, count) : (count + passes - 1) / passes;
+    // Without checkpoints one pass holds every envelope.
+    p->chunk = chunk > 0              ? std::min(chunk, count)
+               : checkpoint_every > 0 ? qhk::bpm_default_chunk(n, count)
+                                      : count;
     p->x.reset(static_cast<std::size_t>(nz) * n * n);
     p->plan = std::make_unique<qhk::BpmPlan>(p->tables, p->chunk, checkpoint_every == 0, checkpoint_every);
     *plan = p.release();

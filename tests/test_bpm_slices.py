@@ -39,12 +39,12 @@ def test_slice_passes_match_the_oracle(cuda, n, count):
 
 
 def test_passes_over_the_views_agree_with_one_pass(cuda):
-    """Enough views that the plan takes them in several passes: fields bitwise those of one pass, the gradient
+    """As many views as the plan takes in two passes: fields bitwise those of one pass, the gradient
     up to the order in which the passes' sums are added (two passes of float32 sums: 4e-7)."""
     from oracle import qh_oracle as O
     from qoraholo_b200.autograd import BpmModel
 
-    n, nz, count = 256, 3, 40  # 73 MB of state
+    n, nz, count = 256, 3, 49  # 86 MB of state
     rng = np.random.default_rng(3)
     il = O.circular_scan(count, 0.9, G)
     ri = cuda.from_numpy((G[1] + 0.03 * rng.random((nz, n, n))).astype(np.float32)).cuda()
@@ -56,3 +56,18 @@ def test_passes_over_the_views_agree_with_one_pass(cuda):
         out.append((y.detach().cpu().numpy(), x.grad.cpu().numpy()))
     assert np.array_equal(out[0][0], out[1][0])
     assert rel_err(out[0][1], out[1][1]) < 4e-7
+
+
+@pytest.mark.parametrize("n,count,passes", [(256, 49, 2), (256, 52, 2), (384, 20, 2),  # 72 to 112 MB of state
+                                            (256, 40, 1), (260, 36, 1),  # halves would make another group of views
+                                            (352, 20, 1), (512, 18, 1), (512, 30, 1),  # below, above, several passes
+                                            (160, 96, 1), (240, 49, 1), (272, 33, 1)])  # small sides, no two radices
+def test_the_default_splits_the_views_only_where_it_pays(cuda, n, count, passes):
+    """By the buffers the plan holds: those of a plan told how many views a pass takes."""
+    from oracle import qh_oracle as O
+    from qoraholo_b200.autograd import BpmPlan
+
+    il = O.circular_scan(count, 0.9, G)
+    plans = [BpmPlan(2, n, il, G, chunk=c, checkpoint_every=1) for c in (0, -(-count // passes), count)]
+    held = [p.device_bytes for p in plans]
+    assert held[0] == held[1] and (held[0] == held[2]) == (passes == 1)
