@@ -220,6 +220,10 @@ int qhk_fft_axis_engine(int engine);
  * [1, 2^126) on the current device. `mismatches` receives their number (0 when the two agree
  * everywhere), `first_bad` the bits of the smallest mismatching input. Synchronous. */
 int qhk_selftest_rcp_sqrt(uint64_t* mismatches, uint32_t* first_bad);
+/* Self-check of the autotuner's timing: times a kernel of 100 us whose launch takes 60 us of host work (1) and
+ * one of 130 us (2). `choice` receives the one it takes for the faster; 1 where host work does not count.
+ * Synchronous. */
+int qhk_selftest_autotune(int* choice);
 /* FGP step form of tv_prox (bitwise the same results): 0 the tuned one, 1 the extrapolated point
  * stored between steps (13 volumes of traffic per step), 2 recomputed from the two previous duals
  * (10 volumes), 3 two steps per pass (13 volumes per two steps; needs rows of a multiple of 4

@@ -126,6 +126,7 @@ _PROTOS = {
     "qhk_autotune_enable": (_I, [_I]),
     "qhk_autotune_radix": (_I, [_I]),
     "qhk_fft_axis_engine": (_I, [_I]),
+    "qhk_selftest_autotune": (_I, [C.POINTER(_I)]),
     "qhk_selftest_rcp_sqrt": (_I, [C.POINTER(C.c_uint64), C.POINTER(C.c_uint32)]),
     "qhk_tv_form": (_I, [_I]),
     "qhk_autotune_report": (C.c_size_t, [_VP, C.c_size_t]),
@@ -323,6 +324,14 @@ def selftest_rcp_sqrt():
     n, b = C.c_uint64(), C.c_uint32()
     check(lib().qhk_selftest_rcp_sqrt(C.byref(n), C.byref(b)))
     return n.value, b.value
+
+
+def selftest_autotune() -> int:
+    """The autotuner's choice between a kernel of 100 us behind 60 us of host work (1) and one of 130 us (2)
+    (qhk_selftest_autotune)."""
+    choice = _I()
+    check(lib().qhk_selftest_autotune(C.byref(choice)))
+    return choice.value
 
 
 def synthesize_holograms_device(d_ratio, count, n, illuminations, pixel, carrier=(5.0, 5.0), reference_amplitude=1.0,

@@ -105,40 +105,59 @@ bool is_tuned(const TuneKey& key) {
 bool autotune_enabled() { return g_enabled.load() != 0; }
 void set_autotune_enabled(bool on) { g_enabled.store(on ? 1 : 0); }
 
+int fastest_candidate(const std::vector<int>& candidates, const std::function<void(int)>& run, cudaStream_t s,
+                      std::vector<std::pair<int, float>>* timings) {
+  // The candidates take turns, and each counts with its fastest turn: timed one after another, the first ones saw
+  // clocks still rising (y passes of 150 x 180^2 came out at 9.5 or at 13 us from one plan to the next). A turn is
+  // an untimed launch and two timed ones behind it: the untimed one leaves L2 as a run of the same candidate
+  // does, and while it runs the host prepares the next, whose occupancy query and tensor maps would otherwise
+  // count, as the start of a lone launch does (an FGP pair of 64^3 19.5 us instead of 15.9; with lone launches two
+  // plans in three of 4 x 64^3 FISTA-TV took the form whose solve is 1.53 ms instead of the one of 1.43). After
+  // the first turn only candidates within half of the fastest go on, so that plans run the slow ones no oftener
+  // than before.
+  constexpr int kTurns = 3, kTimed = 2;
+  constexpr float kStillIn = 1.5f;
+  Event start, stop;
+  timings->clear();
+  for (const int c : candidates) {
+    run(c);
+    timings->emplace_back(c, 0.0f);
+  }
+  float best = 0.0f;
+  int choice = candidates.front();
+  for (int turn = 0; turn < kTurns; ++turn) {
+    const float limit = kStillIn * best;  // of the turns before
+    for (auto& [c, us] : *timings) {
+      if (turn > 0 && us > limit) continue;
+      run(c);
+      start.record(s);
+      for (int r = 0; r < kTimed; ++r) run(c);
+      stop.record(s);
+      check(cudaEventSynchronize(stop.get()), "autotune");
+      const float t = 1000.0f * stop.since(start) / kTimed;
+      us = turn == 0 ? t : std::min(us, t);
+      best = best == 0.0f ? us : std::min(best, us);
+    }
+  }
+  float least = 0.0f;
+  for (const auto& [c, us] : *timings) {
+    if (least == 0.0f || us < least) {
+      least = us;
+      choice = c;
+    }
+  }
+  return choice;
+}
+
 int autotune(const TuneKey& key, const std::vector<int>& candidates, int fallback,
-             const std::function<void(int)>& run, cudaStream_t s, int reps) {
+             const std::function<void(int)>& run, cudaStream_t s) {
   if (!autotune_enabled() || candidates.size() < 2) return tuned_choice(key, fallback);
   if (is_tuned(key)) return tuned_choice(key, fallback);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   check(cudaStreamIsCapturing(s, &cap), "cudaStreamIsCapturing");
   if (cap != cudaStreamCaptureStatusNone) return tuned_choice(key, fallback);
-  Event start, stop;
   Entry e;
-  float best = 0;
-  // The candidates take turns, and each counts with its fastest turn: timed one after another, the first ones
-  // saw clocks still rising (y passes of 150 x 180^2 came out at 9.5 or at 13 us from one plan to the next).
-  constexpr int kTurns = 3;
-  const int each = std::max(1, (reps + kTurns - 1) / kTurns);
-  for (const int c : candidates) {
-    run(c);
-    e.timings.emplace_back(c, 0.0f);
-  }
-  for (int turn = 0; turn < kTurns; ++turn) {
-    for (auto& [c, us] : e.timings) {
-      start.record(s);
-      for (int r = 0; r < each; ++r) run(c);
-      stop.record(s);
-      check(cudaEventSynchronize(stop.get()), "autotune");
-      const float t = 1000.0f * stop.since(start) / static_cast<float>(each);
-      us = turn == 0 ? t : std::min(us, t);
-    }
-  }
-  for (const auto& [c, us] : e.timings) {
-    if (best == 0 || us < best) {
-      best = us;
-      e.choice = c;
-    }
-  }
+  e.choice = fastest_candidate(candidates, run, s, &e.timings);
   std::lock_guard<std::mutex> lk(g_tune_mutex);
   const auto ins = g_tuned.emplace(key, std::move(e));
   if (ins.second) append_table(key, ins.first->second.choice);

@@ -2,8 +2,8 @@
 // fastest per (device, family, shape), for the rest of the process.
 //
 // Tuning runs when a plan is built (never inside a stream capture): each candidate is launched on
-// the plan's own scratch buffers, once to warm up and then in turns, `reps` times in all, between CUDA events, and
-// the candidate with the smallest time wins. Kernels then read their shape from the table, falling
+// the plan's own scratch buffers, once to warm up and then in turns between CUDA events, and the candidate with
+// the smallest time wins. Kernels then read their shape from the table, falling
 // back to a fixed heuristic when a shape was never tuned (or tuning is off: QHK_AUTOTUNE=0). With
 // QHK_AUTOTUNE_FILE set, choices are also read from and appended to that file, so that another run
 // (a profiled one, say) uses the same shapes without timing them again. The tile-shape choices only
@@ -16,6 +16,7 @@
 #include <array>
 #include <functional>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "qhk_util.cuh"
@@ -49,7 +50,15 @@ void set_autotune_enabled(bool on);
 // a tuned key is not timed again). No-op, returning the fallback, when tuning is off, the key has
 // a single candidate or s is capturing. Returns the choice in effect.
 int autotune(const TuneKey& key, const std::vector<int>& candidates, int fallback,
-             const std::function<void(int)>& run, cudaStream_t s, int reps = 3);
+             const std::function<void(int)>& run, cudaStream_t s);
+
+// The timing by itself, without the table: the fastest candidate, and the microseconds of each.
+int fastest_candidate(const std::vector<int>& candidates, const std::function<void(int)>& run, cudaStream_t s,
+                      std::vector<std::pair<int, float>>* timings);
+
+// fastest_candidate on two kernels that only wait: candidate 1 for 100 us, after 60 us of host work per launch,
+// and candidate 2 for 130 us. Returns the choice, 1 where the host's work does not count.
+int selftest_autotune();
 
 // One line per tuned key: family, shape, choice, and the time of every candidate in microseconds.
 std::string autotune_report();

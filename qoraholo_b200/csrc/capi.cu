@@ -819,6 +819,13 @@ int qhk_selftest_rcp_sqrt(uint64_t* mismatches, uint32_t* first_bad) {
   });
 }
 
+int qhk_selftest_autotune(int* choice) {
+  return guard([&] {
+    qhk::require(choice, "selftest_autotune: null argument");
+    *choice = qhk::selftest_autotune();
+  });
+}
+
 int qhk_fft_axis_engine(int engine) {
   return guard([&] {
     qhk::require(engine >= -1 && engine <= 2, "fft_axis_engine: -1, 0, 1 or 2");

@@ -1,8 +1,11 @@
-// Device self-checks of arithmetic helpers that restate IEEE operations with other instructions: every
+// Device self-checks. Of arithmetic helpers that restate IEEE operations with other instructions: every
 // input of the helper's domain is run through it and through the IEEE intrinsics it replaces, and the
-// mismatches are counted (qhk_selftest_rcp_sqrt).
+// mismatches are counted (qhk_selftest_rcp_sqrt). Of the autotuner's timing, on kernels of known duration
+// (qhk_selftest_autotune).
+#include <chrono>
 #include <cstdint>
 
+#include "autotune.hpp"
 #include "qhk_internal.hpp"
 #include "rcp_sqrt2.cuh"
 
@@ -29,7 +32,34 @@ __global__ void k_check_rcp_sqrt(std::uint32_t first, std::uint32_t last, float 
   }
 }
 
+// Returns after `ns` nanoseconds, or after a million looks at the clock.
+__global__ void k_wait(unsigned ns) {
+  unsigned long long first, now;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(first));
+  for (int i = 0; i < 1000000; ++i) {
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+    if (now - first >= ns) break;
+  }
+}
+
 }  // namespace
+
+int selftest_autotune() {
+  Stream stream;
+  std::vector<std::pair<int, float>> timings;
+  const auto run = [&](int c) {
+    if (c == 1) {
+      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(60);
+      while (std::chrono::steady_clock::now() < until) {
+      }
+    }
+    k_wait<<<1, 1, 0, stream.get()>>>(c == 1 ? 100000u : 130000u);
+    check_launch("selftest autotune");
+  };
+  const int choice = fastest_candidate({2, 1}, run, stream.get(), &timings);
+  check(cudaStreamSynchronize(stream.get()), "selftest autotune");
+  return choice;
+}
 
 void selftest_rcp_sqrt(unsigned long long* mismatches, unsigned* first_bad) {
   DevBuf<unsigned long long> bad(1);

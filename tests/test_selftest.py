@@ -1,4 +1,5 @@
-"""Device self-checks of arithmetic that restates IEEE operations with other instructions."""
+"""Device self-checks of arithmetic that restates IEEE operations with other instructions, and of the autotuner's
+timing."""
 
 from __future__ import annotations
 
@@ -14,3 +15,11 @@ def test_projection_factor_equals_ieee_sqrt_and_reciprocal_everywhere(cuda):
 
     mismatches, first = capi.selftest_rcp_sqrt()
     assert mismatches == 0, f"{mismatches} mismatches, first at x bits {first:#010x}"
+
+
+def test_the_autotuner_times_the_device_and_not_the_host(cuda):
+    """A kernel of 100 us behind 60 us of host work is faster than one of 130 us: a solve queues its launches, so
+    the host's work runs while the kernel before does."""
+    from qoraholo_b200 import capi
+
+    assert capi.selftest_autotune() == 1
