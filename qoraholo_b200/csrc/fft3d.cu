@@ -9,6 +9,7 @@
 //     value) with the split / merge step in shared memory;
 //   * complex rows, with the clamp of the complex GP loop between its inverse and forward row
 //     transforms, or the refractive index as the epilogue of the last inverse.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
@@ -698,8 +699,10 @@ TuneKey axis_key(int n_outer, std::size_t so, int n, std::size_t sp, int ni, boo
 
 namespace {
 
-// Engine of an axis pass (FFT decomposition): 1 and 2 the register engine's variants, 0 the staged
-// engine with its own tile width.
+// Engine of an axis pass (FFT decomposition): 1 and 2 the register engine's variants, 3 the two-factor engine
+// and 0 the staged engine, these two with tile widths of their own.
+constexpr int kTwoEngine = 3;
+
 TuneKey engine_key(int n_outer, std::size_t so, int n, std::size_t sp, int ni, bool forward, AxisMode mode,
                    int batch) {
   return tune_key(TuneFamily::axis_engine,
@@ -726,23 +729,38 @@ bool radix_tuning_enabled() {
 
 void set_radix_tuning(bool on) { g_radix_tuning.store(on ? 1 : 0, std::memory_order_relaxed); }
 
+namespace {
+
+// The engine where nothing is forced or tuned. 192 and 512 on the register engine hold 24 and 32 values a thread;
+// without the restore the two-factor engine is faster (192^3: y pass 12 us against 17; 512^3: 208 against 296,
+// from_data 265 against 317; with it 23 against 21 and 527 against 512).
+int default_axis_engine(int n, AxisMode mode) {
+  const bool restore = mode == AxisMode::restore_half || mode == AxisMode::restore_mask;
+  if ((n == 192 || n == 512) && !restore && axis_two_covers(n)) return kTwoEngine;
+  if (axis_reg_variants(n) > 0) return 1;
+  return axis_two_covers(n) ? kTwoEngine : 0;
+}
+
+// The engine of a pass, for the launch and for the tuner alike.
+int axis_engine(int n_outer, std::size_t so, int n, std::size_t sp, int ni, bool forward, AxisMode mode, int batch) {
+  const int forced = g_axis_engine.load(std::memory_order_relaxed);
+  const int variants = axis_reg_variants(n);
+  if (forced == 0) return 0;
+  if (forced > 0 && variants > 0) return std::min(forced, variants);
+  const int engine = default_axis_engine(n, mode);
+  if (variants == 0 || !radix_tuning_enabled()) return engine;
+  return tuned_choice(engine_key(n_outer, so, n, sp, ni, forward, mode, batch), engine);
+}
+
+}  // namespace
+
 void axis_pass(float2* data, int n_outer, std::size_t so, int n, std::size_t sp, int ni, bool forward,
                AxisMode mode, float scale, const AxisAux& aux, cudaStream_t s, int batch, std::size_t sb) {
   require(n_outer >= 1 && n_outer <= 65535 && batch >= 1 && batch <= 65535,
           "fft: too many lines in the outer dimension");
-  const int forced = g_axis_engine.load(std::memory_order_relaxed);
-  int engine = 1;
-  if (forced >= 0 && forced <= axis_reg_variants(n)) {
-    engine = forced;
-  } else if (axis_reg_variants(n) > 0 && radix_tuning_enabled()) {
-    engine = tuned_choice(engine_key(n_outer, so, n, sp, ni, forward, mode, batch), 1);
-  }
-  // 192 and 512 on the register engine hold 24 and 32 values a thread; without the restore the two-factor engine is
-  // faster (192^3: y pass 12 us against 17; 512^3: 208 against 296, from_data 265 against 317; with it 23 against
-  // 21 and 527 against 512).
-  const bool restore = mode == AxisMode::restore_half || mode == AxisMode::restore_mask;
-  const bool two = forced < 0 && (n == 192 || n == 512) && !restore && axis_two_covers(n) && !radix_tuning_enabled();
-  if (!two && engine != 0 && axis_pass_reg(data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb, engine)) {
+  const int engine = axis_engine(n_outer, so, n, sp, ni, forward, mode, batch);
+  if (engine != 0 && engine != kTwoEngine &&
+      axis_pass_reg(data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb, engine)) {
     return;
   }
   if (engine != 0 && axis_two_covers(n)) {
@@ -759,25 +777,31 @@ void tune_axis_pass(float2* data, int n_outer, std::size_t so, int n, std::size_
                     AxisMode mode, float scale, const AxisAux& aux, cudaStream_t s, int batch, std::size_t sb) {
   require(n_outer >= 1 && n_outer <= 65535 && batch >= 1 && batch <= 65535,
           "fft: too many lines in the outer dimension");
-  if (const int variants = axis_reg_variants(n); variants > 0) {
-    // The register engine covers n: its decomposition is fixed unless radix tuning is on, in which case
-    // its variants and the staged engine (at its default tile width) are timed against each other.
-    if (!radix_tuning_enabled()) return;
+  if (const int variants = axis_reg_variants(n); variants > 0 && radix_tuning_enabled()) {
+    // The register engine's variants, the default engine where that is another one, and the staged engine, the
+    // latter two at their default tile widths.
+    const int fallback = default_axis_engine(n, mode);
     std::vector<int> candidates{1};
     if (variants > 1) candidates.push_back(2);
+    if (fallback == kTwoEngine) candidates.push_back(kTwoEngine);
     if (static_cast<std::size_t>(n) * 2 * sizeof(float2) <= 200 * 1024) candidates.push_back(0);
-    autotune(engine_key(n_outer, so, n, sp, ni, forward, mode, batch), candidates, 1,
+    autotune(engine_key(n_outer, so, n, sp, ni, forward, mode, batch), candidates, fallback,
              [&](int c) {
                if (c == 0) {
                  axis_cols(axis_default(n), data, n_outer, so, n, sp, ni, forward, mode, scale, aux, batch, sb, s);
+               } else if (c == kTwoEngine) {
+                 axis_pass_two(axis_two_columns(n).front(), data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s,
+                               batch, sb);
                } else {
                  axis_pass_reg(data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb, c);
                }
              },
              s);
-    return;
   }
-  if (axis_two_covers(n)) {
+  const int engine = axis_engine(n_outer, so, n, sp, ni, forward, mode, batch);
+  // No tile width to choose on the register engine; the staged one keeps its default where it is not the only one.
+  if (engine == 1 || engine == 2 || (engine == 0 && axis_reg_variants(n) > 0)) return;
+  if (engine == kTwoEngine) {
     autotune(axis_key(n_outer, so, n, sp, ni, forward, mode, batch), axis_two_columns(n),
              axis_two_columns(n).front(), [&](int c) {
                axis_pass_two(c, data, n_outer, so, n, sp, ni, forward, mode, scale, aux, s, batch, sb);

@@ -434,6 +434,11 @@ OdtPlan::OdtPlan(const OdtConfig& cfg, const float* illum_fyfx) : cfg_(cfg) {
   tune();
 }
 
+// Real GP steps as a plane pass each between two z passes (solve_real).
+bool OdtPlan::planes_on_chip() const {
+  return real_ && !cfg_.tv && cfg_.iterations > 0 && plane_gp_covers(cfg_.grid.n);
+}
+
 // Autotunes the launch shapes of this plan's passes on its own buffers (scratch at this point):
 // the axis passes' tile widths and the FGP tile height (autotune.hpp). Results do not depend on
 // the shapes chosen.
@@ -457,6 +462,7 @@ void OdtPlan::tune() {
     check(cudaMemsetAsync(a_.get(), 0, a_.bytes(), s), "cudaMemset");
     check(cudaMemsetAsync(hits_.get(), 0, hits_.bytes(), s), "cudaMemset");
     for (const bool fwd : {true, false}) {
+      if (fwd && planes_on_chip()) continue;  // no such pass
       tune_axis_pass(scratch, b * nz, nh, n, h, h, fwd, AxisMode::plain, 1.0f, AxisAux{}, s);
     }
     tune_axis_pass(scratch, 1, nh, nz, nh, static_cast<int>(nh), false, AxisMode::from_data, 1.0f, aux, s, b, half_);
@@ -536,7 +542,7 @@ void OdtPlan::solve_real(float* index, float inv, cudaStream_t s) {
   // tiles straddle its rows, so none is ragged and all start on a 128-byte boundary (256^3, 129 bins per row:
   // 47 us for the pass with the restore, from 53).
   axis_pass(e, 1, nh, nz, nh, static_cast<int>(nh), false, AxisMode::from_data, inv, aux, s, b, half_);
-  if (!cfg_.tv && cfg_.iterations > 0 && plane_gp_covers(n)) {
+  if (planes_on_chip()) {
     // GP with whole planes on chip: each step is a plane pass (inverse y, C2R, clamp, R2C, forward y) and a
     // z pass with the restore.
     for (int it = 0; it < cfg_.iterations; ++it) {

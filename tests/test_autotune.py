@@ -85,3 +85,43 @@ def test_radix_tuning_times_the_decompositions(cuda):
     plain = _run(cuda, capi, 64, 80, options)
     assert "axis_engine" in capi.autotune_report()
     assert rel_err(tuned - G[1], plain - G[1]) < 1e-5
+
+
+def _axis_line(capi, family, n, nz, forward):
+    """The report's line of the plain y pass of half-spectrum planes (nz, n, n / 2 + 1), or None."""
+    h = n // 2 + 1
+    key = f"{family} device 0 shape {n} {h} {nz} {n * h} {h} {16 + int(forward)} "
+    return next((line for line in capi.autotune_report().splitlines() if line.startswith(key)), None)
+
+
+@pytest.mark.parametrize("n", [192, 512])
+def test_the_tuner_times_the_engine_that_runs(cuda, n):
+    """The passes of 192 and 512 without the restore run on the two-factor engine: its tile widths are timed where it
+    has a choice (192), and it is a candidate where the decomposition is tuned."""
+    from qoraholo_b200 import capi
+
+    options = dict(iterations=1, solver="tv", tv_inner=1)
+    plain = _run(cuda, capi, n, 10, options)
+    for forward in (True, False):
+        line = _axis_line(capi, "axis_cols", n, 10, forward)
+        assert (line is not None and "16: " in line and "8: " in line) if n == 192 else line is None
+    try:
+        capi.autotune_radix(True)
+        tuned = _run(cuda, capi, n, 14, options)
+    finally:
+        capi.autotune_radix(False)
+    for forward in (True, False):
+        line = _axis_line(capi, "axis_engine", n, 14, forward)
+        assert line is not None and all(f"{c}: " in line for c in (1, 3, 0))
+    assert np.isfinite(plain).all() and np.isfinite(tuned).all()
+
+
+def test_no_pass_is_timed_that_does_not_run(cuda):
+    """GP steps with whole planes on chip have no forward y pass."""
+    from qoraholo_b200 import capi
+
+    _run(cuda, capi, 90, 14, dict(iterations=1, solver="gp"))
+    assert _axis_line(capi, "axis_cols", 90, 14, True) is None
+    assert _axis_line(capi, "axis_cols", 90, 14, False) is not None
+    _run(cuda, capi, 90, 18, dict(iterations=1, solver="tv", tv_inner=1))
+    assert _axis_line(capi, "axis_cols", 90, 18, True) is not None
