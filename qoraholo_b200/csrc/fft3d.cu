@@ -211,26 +211,15 @@ void axis_dispatch(float2* data, int n_outer, std::size_t so, int n, std::size_t
   }
 }
 
-// Row transforms with the length known at compile time (MC > 0) or at run time (MC = 0): with
-// MC the index arithmetic of the staging loops is by constants, not runtime divisions.
-template <bool Fwd, int COLS, int MC>
-__device__ __forceinline__ float2* row_fft(float2* a, float2* b, int cp, const FftLen& L, int tid, int nth) {
-  if constexpr (MC > 0) {
-    return fftdev::passes_fixed<MC, 0, 1, Fwd, COLS>(a, b, cp, L.tw, tid, nth);
-  } else {
-    return smem_fft_cols<Fwd, COLS>(a, b, cp, L, tid, nth);
-  }
-}
-
 // ---- real rows <-> half spectra -----------------------------------------------------------------
 
-template <bool Clamp, int COLS, int MC>
+template <bool Clamp, int COLS>
 __global__ void __launch_bounds__(kThreads)
     k_rows_r2c(const float* __restrict__ x, float2* __restrict__ e, std::size_t rows, int nx, FftLen Lm,
                const float2* __restrict__ twn) {
   extern __shared__ float2 sm[];
   constexpr int cp = COLS + 1;
-  const int M = MC > 0 ? MC : Lm.n;
+  const int M = Lm.n;
   const int h = M + 1;
   float2* A = sm;
   float2* B = sm + static_cast<std::size_t>(h) * cp;
@@ -250,7 +239,7 @@ __global__ void __launch_bounds__(kThreads)
     A[m * cp + row] = v;
   }
   __syncthreads();
-  const float2* res = row_fft<true, COLS, MC>(A, B, cp, Lm, tid, nth);
+  const float2* res = smem_fft_cols<true, COLS>(A, B, cp, Lm, tid, nth);
 
   for (int idx = tid; idx < h * COLS; idx += nth) {
     const int row = idx / h;
@@ -266,13 +255,13 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-template <int Mode, int COLS, int MC>
+template <int Mode, int COLS>
 __global__ void __launch_bounds__(kThreads)
     k_rows_c2r(const float2* __restrict__ e, float* __restrict__ x, std::size_t rows, int nx, FftLen Lm,
                const float2* __restrict__ twn, float nm2, float inv_k02) {
   extern __shared__ float2 sm[];
   constexpr int cp = COLS + 1;
-  const int M = MC > 0 ? MC : Lm.n;
+  const int M = Lm.n;
   const int h = M + 1;
   float2* A = sm;
   float2* B = sm + static_cast<std::size_t>(h) * cp;
@@ -303,7 +292,7 @@ __global__ void __launch_bounds__(kThreads)
     B[k * cp + row] = make_float2(sv.x - t.y, sv.y + t.x);     // sv + i t
   }
   __syncthreads();
-  const float2* res = row_fft<false, COLS, MC>(B, A, cp, Lm, tid, nth);
+  const float2* res = smem_fft_cols<false, COLS>(B, A, cp, Lm, tid, nth);
 
   for (int idx = tid; idx < M * COLS; idx += nth) {
     const int row = idx / M;
@@ -322,12 +311,12 @@ __global__ void __launch_bounds__(kThreads)
 // going through HBM. The operations are those of k_rows_c2r (store) followed by k_rows_r2c (Clamp)
 // on the same values, so the half spectra are bitwise the same. Each CTA reads all its rows before
 // it writes any, so `e` is updated in place.
-template <int COLS, int MC>
+template <int COLS>
 __global__ void __launch_bounds__(kThreads)
     k_rows_c2r_r2c(float2* __restrict__ e, std::size_t rows, FftLen Lm, const float2* __restrict__ twn) {
   extern __shared__ float2 sm[];
   constexpr int cp = COLS + 1;
-  const int M = MC > 0 ? MC : Lm.n;
+  const int M = Lm.n;
   const int h = M + 1;
   float2* A = sm;
   float2* B = sm + static_cast<std::size_t>(h) * cp;
@@ -358,7 +347,7 @@ __global__ void __launch_bounds__(kThreads)
     B[k * cp + row] = make_float2(sv.x - t.y, sv.y + t.x);     // sv + i t
   }
   __syncthreads();
-  float2* real = row_fft<false, COLS, MC>(B, A, cp, Lm, tid, nth);  // real samples 2m, 2m+1 of each row
+  float2* real = smem_fft_cols<false, COLS>(B, A, cp, Lm, tid, nth);  // real samples 2m, 2m+1 of each row
   for (int idx = tid; idx < M * COLS; idx += nth) {
     const int row = idx / M;
     const int m = idx - row * M;
@@ -370,7 +359,7 @@ __global__ void __launch_bounds__(kThreads)
     real[m * cp + row] = v;
   }
   __syncthreads();
-  const float2* res = row_fft<true, COLS, MC>(real, real == A ? B : A, cp, Lm, tid, nth);
+  const float2* res = smem_fft_cols<true, COLS>(real, real == A ? B : A, cp, Lm, tid, nth);
 
   for (int idx = tid; idx < h * COLS; idx += nth) {
     const int row = idx / h;
@@ -391,7 +380,7 @@ __global__ void __launch_bounds__(kThreads)
 // the FISTA point y = x + m (x - xprev), xprev <- x, and the R2C of y's rows into the half spectra e,
 // y itself never written to HBM. Each row r = z * ny + y of the volume (dense (nz, ny, 2M)) is one
 // column of the tile; its divergence reads p_z of plane z - 1 and p_y of row y - 1 from HBM (L2).
-template <int COLS, int MC>
+template <int COLS>
 __global__ void __launch_bounds__(kThreads)
     k_rows_tv_final_r2c(const float* __restrict__ b, const float* __restrict__ pz, const float* __restrict__ py,
                         const float* __restrict__ px, int nz, int ny, float lambda, float momentum,
@@ -399,7 +388,7 @@ __global__ void __launch_bounds__(kThreads)
                         const float2* __restrict__ twn) {
   extern __shared__ float2 sm[];
   constexpr int cp = COLS + 1;
-  const int M = MC > 0 ? MC : Lm.n;
+  const int M = Lm.n;
   const int h = M + 1;
   const int nx = 2 * M;
   const std::size_t nxy = static_cast<std::size_t>(nx) * ny;
@@ -454,7 +443,7 @@ __global__ void __launch_bounds__(kThreads)
     A[m * cp + row] = v;
   }
   __syncthreads();
-  const float2* res = row_fft<true, COLS, MC>(A, B, cp, Lm, tid, nth);
+  const float2* res = smem_fft_cols<true, COLS>(A, B, cp, Lm, tid, nth);
 
   for (int idx = tid; idx < h * COLS; idx += nth) {
     const int row = idx / h;
@@ -472,13 +461,13 @@ __global__ void __launch_bounds__(kThreads)
 
 // ---- complex rows -----------------------------------------------------------------------------------
 
-template <bool Fwd, int Mode, int COLS, int NC>
+template <bool Fwd, int Mode, int COLS>
 __global__ void __launch_bounds__(kThreads)
     k_rows_c2c(float2* __restrict__ data, std::size_t rows, FftLen L, float scale, float* __restrict__ index,
                float nm2, float inv_k02) {
   extern __shared__ float2 sm[];
   constexpr int cp = COLS + 1;
-  const int n = NC > 0 ? NC : L.n;
+  const int n = L.n;
   float2* A = sm;
   float2* B = sm + static_cast<std::size_t>(n) * cp;
   const std::size_t r0 = static_cast<std::size_t>(blockIdx.x) * COLS;
@@ -494,9 +483,9 @@ __global__ void __launch_bounds__(kThreads)
   __syncthreads();
   float2* res;
   if constexpr (Mode == static_cast<int>(RowMode::plain)) {
-    res = row_fft<Fwd, COLS, NC>(A, B, cp, L, tid, nth);
+    res = smem_fft_cols<Fwd, COLS>(A, B, cp, L, tid, nth);
   } else {
-    res = row_fft<false, COLS, NC>(A, B, cp, L, tid, nth);
+    res = smem_fft_cols<false, COLS>(A, B, cp, L, tid, nth);
     if constexpr (Mode == static_cast<int>(RowMode::inv_clamp_fwd)) {
       float2* other = res == A ? B : A;
       for (int idx = tid; idx < n * COLS; idx += nth) {
@@ -506,7 +495,7 @@ __global__ void __launch_bounds__(kThreads)
         res[pos * cp + row] = make_float2(fmaxf(v.x * scale, 0.0f), 0.0f);
       }
       __syncthreads();
-      res = row_fft<true, COLS, NC>(res, other, cp, L, tid, nth);
+      res = smem_fft_cols<true, COLS>(res, other, cp, L, tid, nth);
     }
   }
   for (int idx = tid; idx < n * COLS; idx += nth) {
@@ -531,7 +520,7 @@ constexpr int rows_per_cta(int n) {
   return c;
 }
 
-template <int COLS, int MC>
+template <int COLS>
 void launch_r2c(const float* x, float2* e, std::size_t rows, int nx, bool clamp, cudaStream_t s) {
   const int M = nx / 2;
   const FftLen& Lm = fft_len(M);
@@ -539,16 +528,16 @@ void launch_r2c(const float* x, float2* e, std::size_t rows, int nx, bool clamp,
   const std::size_t smem = 2 * static_cast<std::size_t>(M + 1) * (COLS + 1) * sizeof(float2);
   const unsigned grid = static_cast<unsigned>((rows + COLS - 1) / COLS);
   if (clamp) {
-    allow_smem(k_rows_r2c<true, COLS, MC>, smem);
-    k_rows_r2c<true, COLS, MC><<<grid, kThreads, smem, s>>>(x, e, rows, nx, Lm, Ln.tw);
+    allow_smem(k_rows_r2c<true, COLS>, smem);
+    k_rows_r2c<true, COLS><<<grid, kThreads, smem, s>>>(x, e, rows, nx, Lm, Ln.tw);
   } else {
-    allow_smem(k_rows_r2c<false, COLS, MC>, smem);
-    k_rows_r2c<false, COLS, MC><<<grid, kThreads, smem, s>>>(x, e, rows, nx, Lm, Ln.tw);
+    allow_smem(k_rows_r2c<false, COLS>, smem);
+    k_rows_r2c<false, COLS><<<grid, kThreads, smem, s>>>(x, e, rows, nx, Lm, Ln.tw);
   }
   check_launch("rows r2c");
 }
 
-template <int COLS, int MC>
+template <int COLS>
 void launch_tv_final_r2c(const float* b, const float* const p[3], int nz, int ny, int nx, float lambda,
                          float momentum, float* xprev, float2* e, cudaStream_t s) {
   const int M = nx / 2;
@@ -557,25 +546,25 @@ void launch_tv_final_r2c(const float* b, const float* const p[3], int nz, int ny
   const std::size_t rows = static_cast<std::size_t>(nz) * ny;
   const std::size_t smem = 2 * static_cast<std::size_t>(M + 1) * (COLS + 1) * sizeof(float2);
   const unsigned grid = static_cast<unsigned>((rows + COLS - 1) / COLS);
-  allow_smem(k_rows_tv_final_r2c<COLS, MC>, smem);
-  k_rows_tv_final_r2c<COLS, MC><<<grid, kThreads, smem, s>>>(b, p[0], p[1], p[2], nz, ny, lambda, momentum, xprev,
+  allow_smem(k_rows_tv_final_r2c<COLS>, smem);
+  k_rows_tv_final_r2c<COLS><<<grid, kThreads, smem, s>>>(b, p[0], p[1], p[2], nz, ny, lambda, momentum, xprev,
                                                               e, rows, Lm, Ln.tw);
   check_launch("rows tv final r2c");
 }
 
-template <int COLS, int MC>
+template <int COLS>
 void launch_c2r_r2c(float2* e, std::size_t rows, int nx, cudaStream_t s) {
   const int M = nx / 2;
   const FftLen& Lm = fft_len(M);
   const FftLen& Ln = fft_len(nx);
   const std::size_t smem = 2 * static_cast<std::size_t>(M + 1) * (COLS + 1) * sizeof(float2);
   const unsigned grid = static_cast<unsigned>((rows + COLS - 1) / COLS);
-  allow_smem(k_rows_c2r_r2c<COLS, MC>, smem);
-  k_rows_c2r_r2c<COLS, MC><<<grid, kThreads, smem, s>>>(e, rows, Lm, Ln.tw);
+  allow_smem(k_rows_c2r_r2c<COLS>, smem);
+  k_rows_c2r_r2c<COLS><<<grid, kThreads, smem, s>>>(e, rows, Lm, Ln.tw);
   check_launch("rows c2r r2c");
 }
 
-template <int COLS, int MC>
+template <int COLS>
 void launch_c2r(const float2* e, float* x, std::size_t rows, int nx, C2rMode mode, float nm2, float inv_k02,
                 cudaStream_t s) {
   const int M = nx / 2;
@@ -584,43 +573,43 @@ void launch_c2r(const float2* e, float* x, std::size_t rows, int nx, C2rMode mod
   const std::size_t smem = 2 * static_cast<std::size_t>(M + 1) * (COLS + 1) * sizeof(float2);
   const unsigned grid = static_cast<unsigned>((rows + COLS - 1) / COLS);
   if (mode == C2rMode::index) {
-    allow_smem(k_rows_c2r<1, COLS, MC>, smem);
-    k_rows_c2r<1, COLS, MC><<<grid, kThreads, smem, s>>>(e, x, rows, nx, Lm, Ln.tw, nm2, inv_k02);
+    allow_smem(k_rows_c2r<1, COLS>, smem);
+    k_rows_c2r<1, COLS><<<grid, kThreads, smem, s>>>(e, x, rows, nx, Lm, Ln.tw, nm2, inv_k02);
   } else {
-    allow_smem(k_rows_c2r<0, COLS, MC>, smem);
-    k_rows_c2r<0, COLS, MC><<<grid, kThreads, smem, s>>>(e, x, rows, nx, Lm, Ln.tw, nm2, inv_k02);
+    allow_smem(k_rows_c2r<0, COLS>, smem);
+    k_rows_c2r<0, COLS><<<grid, kThreads, smem, s>>>(e, x, rows, nx, Lm, Ln.tw, nm2, inv_k02);
   }
   check_launch("rows c2r");
 }
 
-template <bool Fwd, int Mode, int COLS, int NC>
+template <bool Fwd, int Mode, int COLS>
 void launch_c2c_rows(float2* data, std::size_t rows, int nx, float scale, float* index, float nm2,
                      float inv_k02, cudaStream_t s) {
   const FftLen& L = fft_len(nx);
   const std::size_t smem = 2 * static_cast<std::size_t>(nx) * (COLS + 1) * sizeof(float2);
-  auto kernel = k_rows_c2c<Fwd, Mode, COLS, NC>;
+  auto kernel = k_rows_c2c<Fwd, Mode, COLS>;
   allow_smem(kernel, smem);
   const unsigned grid = static_cast<unsigned>((rows + COLS - 1) / COLS);
   kernel<<<grid, kThreads, smem, s>>>(data, rows, L, scale, index, nm2, inv_k02);
   check_launch("rows c2c");
 }
 
-template <int COLS, int NC>
+template <int COLS>
 void c2c_rows_dispatch(float2* data, std::size_t rows, int nx, bool forward, RowMode mode, float scale,
                        float* index, float nm2, float inv_k02, cudaStream_t s) {
   switch (mode) {
     case RowMode::plain:
       if (forward) {
-        launch_c2c_rows<true, 0, COLS, NC>(data, rows, nx, scale, index, nm2, inv_k02, s);
+        launch_c2c_rows<true, 0, COLS>(data, rows, nx, scale, index, nm2, inv_k02, s);
       } else {
-        launch_c2c_rows<false, 0, COLS, NC>(data, rows, nx, scale, index, nm2, inv_k02, s);
+        launch_c2c_rows<false, 0, COLS>(data, rows, nx, scale, index, nm2, inv_k02, s);
       }
       break;
     case RowMode::inv_clamp_fwd:
-      launch_c2c_rows<false, 1, COLS, NC>(data, rows, nx, scale, index, nm2, inv_k02, s);
+      launch_c2c_rows<false, 1, COLS>(data, rows, nx, scale, index, nm2, inv_k02, s);
       break;
     case RowMode::inv_index:
-      launch_c2c_rows<false, 2, COLS, NC>(data, rows, nx, scale, index, nm2, inv_k02, s);
+      launch_c2c_rows<false, 2, COLS>(data, rows, nx, scale, index, nm2, inv_k02, s);
       break;
   }
 }
@@ -813,20 +802,16 @@ void tune_axis_pass(float2* data, int n_outer, std::size_t so, int n, std::size_
            [&](int c) { axis_cols(c, data, n_outer, so, n, sp, ni, forward, mode, scale, aux, batch, sb, s); }, s);
 }
 
-// The half length beyond the two engines above with compile-time row kernels; others run the run-time ones.
-constexpr int kFixedHalf = 512;
-
 void rows_r2c(const float* x, float2* e, std::size_t rows, int nx, bool clamp, cudaStream_t s) {
   require(nx >= 2 && nx % 2 == 0, "rfft: row length must be even");
   if (rows_r2c_reg(x, e, rows, nx, clamp, s)) return;
   if (rows_r2c_two(x, e, rows, nx, clamp, s)) return;
-  if (nx == 2 * kFixedHalf) return launch_r2c<rows_per_cta(kFixedHalf), kFixedHalf>(x, e, rows, nx, clamp, s);
   switch (rows_per_cta(nx / 2)) {
-    case 16: launch_r2c<16, 0>(x, e, rows, nx, clamp, s); break;
-    case 8: launch_r2c<8, 0>(x, e, rows, nx, clamp, s); break;
-    case 4: launch_r2c<4, 0>(x, e, rows, nx, clamp, s); break;
-    case 2: launch_r2c<2, 0>(x, e, rows, nx, clamp, s); break;
-    default: launch_r2c<1, 0>(x, e, rows, nx, clamp, s); break;
+    case 16: launch_r2c<16>(x, e, rows, nx, clamp, s); break;
+    case 8: launch_r2c<8>(x, e, rows, nx, clamp, s); break;
+    case 4: launch_r2c<4>(x, e, rows, nx, clamp, s); break;
+    case 2: launch_r2c<2>(x, e, rows, nx, clamp, s); break;
+    default: launch_r2c<1>(x, e, rows, nx, clamp, s); break;
   }
 }
 
@@ -835,13 +820,12 @@ void rows_c2r(const float2* e, float* x, std::size_t rows, int nx, C2rMode mode,
   require(nx >= 2 && nx % 2 == 0, "irfft: row length must be even");
   if (rows_c2r_reg(e, x, rows, nx, mode, nm2, inv_k02, s)) return;
   if (rows_c2r_two(e, x, rows, nx, mode, nm2, inv_k02, s)) return;
-  if (nx == 2 * kFixedHalf) return launch_c2r<rows_per_cta(kFixedHalf), kFixedHalf>(e, x, rows, nx, mode, nm2, inv_k02, s);
   switch (rows_per_cta(nx / 2)) {
-    case 16: launch_c2r<16, 0>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
-    case 8: launch_c2r<8, 0>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
-    case 4: launch_c2r<4, 0>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
-    case 2: launch_c2r<2, 0>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
-    default: launch_c2r<1, 0>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
+    case 16: launch_c2r<16>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
+    case 8: launch_c2r<8>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
+    case 4: launch_c2r<4>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
+    case 2: launch_c2r<2>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
+    default: launch_c2r<1>(e, x, rows, nx, mode, nm2, inv_k02, s); break;
   }
 }
 
@@ -849,13 +833,12 @@ void rows_c2r_r2c(float2* e, std::size_t rows, int nx, cudaStream_t s) {
   require(nx >= 2 && nx % 2 == 0, "rfft: row length must be even");
   if (rows_c2r_r2c_reg(e, rows, nx, s)) return;
   if (rows_c2r_r2c_two(e, rows, nx, s)) return;
-  if (nx == 2 * kFixedHalf) return launch_c2r_r2c<rows_per_cta(kFixedHalf), kFixedHalf>(e, rows, nx, s);
   switch (rows_per_cta(nx / 2)) {
-    case 16: launch_c2r_r2c<16, 0>(e, rows, nx, s); break;
-    case 8: launch_c2r_r2c<8, 0>(e, rows, nx, s); break;
-    case 4: launch_c2r_r2c<4, 0>(e, rows, nx, s); break;
-    case 2: launch_c2r_r2c<2, 0>(e, rows, nx, s); break;
-    default: launch_c2r_r2c<1, 0>(e, rows, nx, s); break;
+    case 16: launch_c2r_r2c<16>(e, rows, nx, s); break;
+    case 8: launch_c2r_r2c<8>(e, rows, nx, s); break;
+    case 4: launch_c2r_r2c<4>(e, rows, nx, s); break;
+    case 2: launch_c2r_r2c<2>(e, rows, nx, s); break;
+    default: launch_c2r_r2c<1>(e, rows, nx, s); break;
   }
 }
 
@@ -863,13 +846,12 @@ void rows_tv_final_r2c(const float* b, const float* const p[3], int nz, int ny, 
                        float* xprev, float2* e, cudaStream_t s) {
   require(nx >= 2 && nx % 2 == 0 && nz >= 1 && ny >= 1, "rfft: row length must be even");
   if (rows_tv_final_r2c_two(b, p, nz, ny, nx, lambda, momentum, xprev, e, s)) return;
-  if (nx == 2 * kFixedHalf) return launch_tv_final_r2c<rows_per_cta(kFixedHalf), kFixedHalf>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s);
   switch (rows_per_cta(nx / 2)) {
-    case 16: launch_tv_final_r2c<16, 0>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
-    case 8: launch_tv_final_r2c<8, 0>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
-    case 4: launch_tv_final_r2c<4, 0>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
-    case 2: launch_tv_final_r2c<2, 0>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
-    default: launch_tv_final_r2c<1, 0>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
+    case 16: launch_tv_final_r2c<16>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
+    case 8: launch_tv_final_r2c<8>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
+    case 4: launch_tv_final_r2c<4>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
+    case 2: launch_tv_final_r2c<2>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
+    default: launch_tv_final_r2c<1>(b, p, nz, ny, nx, lambda, momentum, xprev, e, s); break;
   }
 }
 
@@ -877,11 +859,11 @@ void rows_c2c(float2* data, std::size_t rows, int nx, bool forward, RowMode mode
               float nm2, float inv_k02, cudaStream_t s) {
   if (rows_c2c_two(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s)) return;
   switch (rows_per_cta(nx)) {
-    case 16: c2c_rows_dispatch<16, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
-    case 8: c2c_rows_dispatch<8, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
-    case 4: c2c_rows_dispatch<4, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
-    case 2: c2c_rows_dispatch<2, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
-    default: c2c_rows_dispatch<1, 0>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
+    case 16: c2c_rows_dispatch<16>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
+    case 8: c2c_rows_dispatch<8>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
+    case 4: c2c_rows_dispatch<4>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
+    case 2: c2c_rows_dispatch<2>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
+    default: c2c_rows_dispatch<1>(data, rows, nx, forward, mode, scale, index, nm2, inv_k02, s); break;
   }
 }
 

@@ -29,7 +29,7 @@ def test_transforms_of_every_length_class(cuda, n):
         d = cuda.from_numpy(x).cuda()
         capi.fft2d(d.data_ptr(), 3, n, forward, 0.5)
         assert rel_err(d.cpu().numpy(), 0.5 * fft(x.astype(np.complex128))) < 1e-6
-    nz, ny = 6, 9  # an odd number of rows: the last one is transformed alone
+    nz, ny = 6, 9  # 45 rows: the last tile is ragged
     r = rng.standard_normal((nz - 1, ny, n)).astype(np.float32)
     want = np.fft.rfftn(r.astype(np.float64))
     d, h = cuda.from_numpy(r).cuda(), cuda.empty((nz - 1, ny, n // 2 + 1), dtype=cuda.complex64, device="cuda")
@@ -38,6 +38,23 @@ def test_transforms_of_every_length_class(cuda, n):
     back = cuda.empty_like(d)
     h = cuda.from_numpy(want.astype(np.complex64)).cuda()
     capi.irfft3(h.data_ptr(), back.data_ptr(), nz - 1, ny, n, 1.0 / r.size)
+    assert rel_err(back.cpu().numpy(), r) < 1e-6
+
+
+@pytest.mark.parametrize("nx,nz,ny", [(1024, 2, 4), (1024, 2, 7), (1024, 5, 9), (960, 5, 9), (832, 3, 5)])
+def test_real_rows_of_the_longest_lines(cuda, nx, nz, ny):
+    """Rows whose staged tiles shared memory cuts short (half length 512 = 16 x 32: seven lines, not eight), whole
+    and ragged; the bound is the one of the transforms above."""
+    from qoraholo_b200 import capi
+
+    r = np.random.default_rng(nx + ny).standard_normal((nz, ny, nx)).astype(np.float32)
+    want = np.fft.rfftn(r.astype(np.float64))
+    d, h = cuda.from_numpy(r).cuda(), cuda.empty((nz, ny, nx // 2 + 1), dtype=cuda.complex64, device="cuda")
+    capi.rfft3(d.data_ptr(), h.data_ptr(), nz, ny, nx)
+    assert rel_err(h.cpu().numpy(), want) < 1e-6
+    back = cuda.empty_like(d)
+    h = cuda.from_numpy(want.astype(np.complex64)).cuda()
+    capi.irfft3(h.data_ptr(), back.data_ptr(), nz, ny, nx, 1.0 / r.size)
     assert rel_err(back.cpu().numpy(), r) < 1e-6
 
 
