@@ -58,22 +58,37 @@ def test_real_rows_of_the_longest_lines(cuda, nx, nz, ny):
     assert rel_err(back.cpu().numpy(), r) < 1e-6
 
 
-@pytest.mark.parametrize("n", [4, 10, 12, 30, 34, 48, 66, 90, 96, 126, 150, 154, 160, 176, 182, 196, 200, 208, 210, 220,
-                               224, 226, 230])
-def test_gp_planes_against_the_oracle(cuda, n):
-    """GP with whole planes on chip (up to 224: 226 and 230 have no two radices, and 230 would not fit), for
-    every class of x factors; batches of planes that fill the GPU and that do not."""
+def _gp_against_the_oracle(torch, n, nz, amplitude):
     from oracle import qh_oracle as O
     from qoraholo_b200 import capi
 
     il = O.circular_scan(3, 0.9, G)
     rng = np.random.default_rng(n)
-    fields = (rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n))).astype(np.complex64) * 0.05
-    want, _ = O.reconstruct(fields, il, G, nz=4, iterations=2)
-    plan = capi.OdtPlan(n, 3, il, G, nz=4, iterations=2)
-    d, out = cuda.from_numpy(fields).cuda(), cuda.empty(plan.shape, dtype=cuda.float32, device="cuda")
+    fields = (rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n))).astype(np.complex64) * np.float32(amplitude)
+    want, _ = O.reconstruct(fields, il, G, nz=nz, iterations=2)
+    plan = capi.OdtPlan(n, 3, il, G, nz=nz, iterations=2)
+    d, out = torch.from_numpy(fields).cuda(), torch.empty(plan.shape, dtype=torch.float32, device="cuda")
     plan.run(d.data_ptr(), out.data_ptr())
-    cuda.cuda.synchronize()
+    torch.cuda.synchronize()
     plan.close()
     # 1e-5 of the contrast: ten transforms of 1e-6 each, and two steps that do not amplify them.
     assert rel_err(out.cpu().numpy() - G[1], want - G[1]) < 1e-5
+
+
+@pytest.mark.parametrize("n", [4, 10, 12, 30, 34, 48, 66, 90, 96, 126, 150, 154, 160, 176, 182, 196, 200, 208, 210, 220,
+                               224, 226, 230])
+def test_gp_planes_against_the_oracle(cuda, n):
+    """GP with whole planes on chip (up to 224: 226 and 230 have no two radices, and 230 would not fit), for
+    every class of x factors; four planes, in CTAs of 512 threads."""
+    _gp_against_the_oracle(cuda, n, 4, 0.05)
+
+
+@pytest.mark.parametrize("n,nz", [(10, 150), (66, 150), (90, 160), (96, 160),  # four and more planes per SM: 128 threads
+                                  (120, 150), (128, 150), (150, 152), (154, 150), (160, 150),  # two or three: 256
+                                  (182, 150), (224, 150)])  # one, in more than one wave: 512
+def test_gp_planes_that_fill_the_gpu(cuda, n, nz):
+    """More planes than SMs, for each number of planes that an SM holds and so each CTA size. The contrast falls as
+    1 / nz and the index is stored in float32, of spacing 1.2e-7 at 1.337: with 0.05, an rms contrast of 2e-4, storing
+    it alone is a difference of up to 2.4e-4; with 0.5 nz / 4, an rms contrast of 0.07, of 7e-7."""
+    assert nz > cuda.cuda.get_device_properties(0).multi_processor_count
+    _gp_against_the_oracle(cuda, n, nz, 0.5 * nz / 4)
