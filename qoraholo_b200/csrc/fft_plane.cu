@@ -31,8 +31,12 @@ using twofft::Factors;
 
 __host__ __device__ __forceinline__ int plane_pitch(int n) { return (n / 2 + 1) | 1; }
 
+// The thread count that bounds the registers: 96 a thread for the small radices, which five CTAs of 128 threads
+// leave an SM (8 x 96^3: 35 us per step, 39 with the 118 that the compiler would take), 128 for the others.
+constexpr int plane_bound(int max) { return max == twofft::kSmall ? 640 : 512; }
+
 template <int Max>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(plane_bound(Max), 1)
     k_plane_gp(float2* __restrict__ e, int n, Factors fy, Factors fx, const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
   const int h = n / 2 + 1, P = plane_pitch(n), H = n / 2;
