@@ -26,21 +26,21 @@ using twofft::RowLaunch;
 using twofft::RowTile;
 
 // CTAs per SM to leave registers for, at 256 threads each (axis tiles are 16 columns of at most 16 threads or 8
-// columns of at most 32, row tiles 256 threads): three of 80 registers where the radices fit them, two of 128
-// for larger radices and for the restore, whose two transforms spill at 80 (96^3 x 8: 25 us against 29); the
-// restore of second factors up to 24 in three CTAs of 192 threads.
+// columns of at most 32, row tiles 256 threads): three of 80 registers where the radices fit them (the restore of
+// 8 x 96^3 too: 19.1 us, in two CTAs 22.3), two of 128 for larger radices. The restore of second factors up to 24
+// runs in three CTAs of 192 threads (384^3: 196 us, in two of 256 223).
 constexpr int min_blocks(int max) { return max == twofft::kSmall ? 3 : 2; }
 
 constexpr bool restores(int mode) {
   return mode == static_cast<int>(AxisMode::restore_half) || mode == static_cast<int>(AxisMode::restore_mask);
 }
+constexpr int axis_threads(int mode, int max) { return restores(mode) && max == twofft::kMid ? 192 : 256; }
 
 // ---- axis passes ------------------------------------------------------------------------------------
 
 // COLS = 1 << logc consecutive columns of one outer slice per CTA; COLS * R2 threads (R2 >= R1).
 template <bool Fwd, int Mode, int Max>
-__global__ void __launch_bounds__(restores(Mode) && Max == twofft::kMid ? 192 : 256,
-                                  !restores(Mode) ? min_blocks(Max) : Max == twofft::kMid ? 3 : 2)
+__global__ void __launch_bounds__(axis_threads(Mode, Max), axis_threads(Mode, Max) == 192 ? 3 : min_blocks(Max))
     k_axis_two(float2* __restrict__ data, std::size_t so, std::size_t sp, int ni, Factors f, int logc,
                const float2* __restrict__ tw, float scale, const float2* __restrict__ aux_a,
                const std::uint8_t* __restrict__ aux_h, std::size_t sb) {
