@@ -26,8 +26,11 @@ constexpr int kThreads = 256;
 
 // Pass 1. Rows of real holograms (length N), COLS rows per CTA; writes t1[row][j] = H_row(fx),
 // fx = cx + dxlo + j, for j < W (zero if fx is outside [-N/2, N/2)).
+// Six CTAs per SM (40 registers) for tiles of 16 rows, whose lines are short and mostly one long prime sum per
+// thread: 55 x 206^2 810 us against 1645 in four CTAs of 64 registers, 40 x 262^2 1293 against 2641; tiles of fewer rows
+// stay with four (40 x 574^2 755 us, in six 807).
 template <int COLS>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, COLS == 16 ? 6 : 4)
     k_holo_rows(const float* __restrict__ holo, float2* __restrict__ t1, std::size_t rows, int N, FftLen Lm,
                 const float2* __restrict__ twn, int fx0, int W) {
   extern __shared__ float2 sm[];
