@@ -204,7 +204,8 @@ int qhk_unwrap_noalloc(const float* d_wrapped, float* d_unwrapped, int count, in
  * (environment QHK_AUTOTUNE=0 turns it off). */
 int qhk_autotune_enable(int enabled);
 /* Also time the FFT decomposition of the axis passes (the register engine's variants T x V, the staged
- * radix engine and, for 192 and 512 without the restore, the two-factor engine) when plans are built, and keep the fastest. Off by default (environment
+ * radix engine and, for 192 and 512 without the restore, the two-factor engine) when plans are built,
+ * and keep the fastest. Off by default (environment
  * QHK_AUTOTUNE_RADIX=1 turns it on): the decompositions round differently, so with it on results stay
  * within the oracle's tolerance but depend on which variant won -- runs are no longer bitwise
  * reproducible across processes, nor batches bitwise equal to single requests. */

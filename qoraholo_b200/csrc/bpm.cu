@@ -3,7 +3,7 @@
 // and follows the CPU form (src/cpu/bpm.cpp:18-243) and the tables of src/bpm.cpp:10-60.
 //
 // A pass of the model processes a chunk of nb illuminations at once, all planes (nb, n, n). Each
-// slice is two 2D FFTs. For the sides the two-factor line transforms cover a slice is two passes, each
+// slice is two 2D FFTs. For sides from 48 on with two radices (fft_two.cuh) a slice is two passes, each
 // keeping a line of every plane on chip across a transform, the pointwise step and the opposite transform:
 //   forward:  columns [FFT (completing FFT(w)), S = c (q W + (1 - q) S), IFFT] ->
 //             rows [IFFT (completing IFFT(S)), x 1/n^2, store envelope, times the screen e^{i phase x_k},
@@ -76,8 +76,7 @@ struct ColArgs {
   float phase;          // screen phase per unit contrast
   float inv;            // 1 / n^2
   int has_back;         // kSplit: add data (the back-propagated screen term) to g
-  // kSplitInv: also finish the previous slice's gradient (the first plane's blocks, one pixel per thread
-  // position): grad += gscale phase (part[0] + part[1] + ...), when grad is set.
+  // kSplitInv: also finish the previous slice's gradient (add_slice_gradient), when grad is set.
   const float* part;
   int groups;
   float gscale;
@@ -155,17 +154,6 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// One slice of the forward sweep as two passes, each keeping a line of every
-// plane on chip across a transform, the pointwise step and the opposite transform:
-//   column pass (kPropInv): the forward column transform of the row-transformed envelope completes its
-//     2D FFT W; S = c (q W + (1 - q) S) (as the kPropagate epilogue) is stored; the inverse column
-//     transform of S starts the next inverse 2D FFT. kInvOnly applies only the inverse column transform to
-//     S (the first slice of a recomputed segment).
-//   row pass (kScreenFwd): the inverse row transform completes IFFT(S); x 1/n^2, store the envelope, times
-//     the screen (as the kScreen epilogue), then the forward row transform of the next slice's FFT.
-//     kScaleOut ends the sweep: inverse rows and x 1/n^2 only.
-// The inverse 2D FFT thus runs columns first and the forward one rows first; the recomputed segments use
-// the same two passes, so their envelopes are bitwise the forward sweep's.
 // The previous slice's gradient, added by the column pass: grad += gscale phase (part[0] + part[1] + ...),
 // groups in order. The image rows are shared out over the views' CTAs, a few each, so that no CTA of the pass
 // is held up by them; `t` of the `step` threads of column col.
@@ -182,6 +170,17 @@ __device__ __forceinline__ void add_slice_gradient(const ColArgs& a, int n, int 
   }
 }
 
+// One slice of the forward sweep as two passes, each keeping a line of every plane on chip across a transform, the
+// pointwise step and the opposite transform:
+//   column pass (kPropInv): the forward column transform of the row-transformed envelope completes its
+//     2D FFT W; S = c (q W + (1 - q) S) (as the kPropagate epilogue) is stored; the inverse column
+//     transform of S starts the next inverse 2D FFT. kInvOnly applies only the inverse column transform to
+//     S (the first slice of a recomputed segment).
+//   row pass (kScreenFwd): the inverse row transform completes IFFT(S); x 1/n^2, store the envelope, times
+//     the screen (as the kScreen epilogue), then the forward row transform of the next slice's FFT.
+//     kScaleOut ends the sweep: inverse rows and x 1/n^2 only.
+// The inverse 2D FFT thus runs columns first and the forward one rows first; the recomputed segments use
+// the same two passes, so their envelopes are bitwise the forward sweep's.
 enum SliceMode : int { kPropInv = 0, kInvOnly = 1, kScreenFwd = 2, kScaleOut = 3, kSplitInv = 4 };
 
 template <int Mode, int T, int V>
@@ -718,11 +717,11 @@ void slice_gradient_two(const Factors& f, bool forward, float2* data, const floa
 }
 
 // The sides the slice passes cover, and the dispatch: 64, 128 and 256, whose lines have a compile-time form on
-// the register engine (256^2, 49 views: row pass 17 us, adjoint column pass 37 us, gradient pass 26 us, against
-// 26, 55 and 35 on the two-factor engine), take that; the others the two-factor engine (160^2, 24 views, per
-// slice: 9.3 and 6.9 us forward where the four staged passes took 39; the whole gradient of 60 slices 3.9 ms
-// from 8.6). Sides below 48 keep the staged passes: a slice of so small a plane is a few microseconds of launch
-// latency either way.
+// the register engine (256^2, 25 and 24 views: column passes 12.9 and 12.1 us, row pass 9.7 us, gradient pass
+// 16.7 us, against 14.4, 15.6, 12.9 and 25.8 on the two-factor engine), take that; the others the two-factor
+// engine (160^2, 24 views, per slice: 9.2 and 6.8 us forward where the four staged passes took 39; the whole
+// gradient of 60 slices 3.8 ms from 8.6). Sides below 48 keep the staged passes: a slice of so small a plane is a
+// few microseconds of launch latency either way.
 Factors slice_factors(int n) {
   Factors f;
   twofft::factors(n, &f);
@@ -747,7 +746,9 @@ void with_slice_shape(int n, Reg&& reg, Two&& two) {
 }
 
 // Views per group of the row passes (the groups the gradient is summed in).
-int slice_views(int n) { return n == 64 || n == 128 ? regfft::RowTile<8>::R : n == 256 ? regfft::RowTile<16>::R : kSliceViews; }
+int slice_views(int n) {
+  return n == 64 || n == 128 ? regfft::RowTile<8>::R : n == 256 ? regfft::RowTile<16>::R : kSliceViews;
+}
 int slice_groups(int n, int views) { return (views + slice_views(n) - 1) / slice_views(n); }
 
 void slice_cols(int n, int mode, const ColArgs& a, int nb, cudaStream_t s) {
@@ -965,13 +966,13 @@ BpmTablesHost bpm_tables(int n, int nz, const float* il, int count, float wavele
 }
 
 // Two equal passes where one pass's state (spectrum, envelope, propagator and obliquity, 28 bytes per pixel and
-// view, touched by every slice) is more than L2 keeps from slice to slice and half of it is not, and the halves make
-// no more groups of views than the whole. One pass against two, gradients of 16 to 128 slices: 256^2 with 49 views 24.9 and 22.8 ms,
-// with 64 views 16.7 and 16.1; 264^2 and 384^2 with 49 and 20 views 12.3 and 10.0, 7.6 and 6.5; forty sides and counts
-// in this range 1.00 to 1.22 times. Outside it one pass: with another group (256^2, 40 views: 20.1 and 21.6 ms),
-// below 72 MB (352^2, 20 views: 6.0 and 6.6), above 112 MB (480^2, 20 views: 10.4 and 10.8; 512^2, 49 views, nine
-// passes: 17.1 and 20.5), and for sides up to 240, where either can be faster (200^2, 64 views: 8.8 and 7.7; 224^2,
-// 49 views: 6.0 and 6.7).
+// view, touched by every slice) is more than L2 keeps from slice to slice and half of it is not, and the halves
+// make no more groups of views than the whole. One pass against two, gradients of 16 to 128 slices: 256^2 with 49
+// views 24.9 and 22.8 ms, with 64 views 16.7 and 16.1; 264^2 and 384^2 with 49 and 20 views 12.3 and 10.0, 7.6 and
+// 6.5; forty sides and counts in this range 1.00 to 1.22 times. Outside it one pass: with another group (256^2,
+// 40 views: 20.1 and 21.6 ms), below 72 MB (352^2, 20 views: 6.0 and 6.6), above 112 MB (480^2, 20 views: 10.4 and
+// 10.8; 512^2, 49 views, nine passes: 17.1 and 20.5), and for sides up to 240, where either can be faster (200^2, 64
+// views: 8.8 and 7.7; 224^2, 49 views: 6.0 and 6.7).
 int bpm_default_chunk(int n, int count) {
   constexpr std::size_t kViewBytes = 28, kLow = std::size_t{72} << 20, kHigh = std::size_t{112} << 20;
   const std::size_t state = kViewBytes * n * n * count;
@@ -1075,7 +1076,7 @@ void BpmPlan::forward(const float* x, int first, int nb, cudaStream_t s) {
   k_first_screen<<<grid_for(total), kThreads, 0, s>>>(w_.get(), store_on_ ? stored_.get() : nullptr, x, t_.phase,
                                                       plane_, total);
   check_launch("bpm start");
-  // Two passes per slice on the two-factor engine (k_slice_cols / k_slice_rows).
+  // Two passes per slice (slice_cols, slice_rows).
   if (slice_covers(t_.n)) {
     rows_forward(w_.get(), t_.n, nb, s);
     for (int k = 0; k < nz; ++k) {
@@ -1150,8 +1151,8 @@ void BpmPlan::adjoint(const float* x, const float2* residual_or_null, int first,
     }
     return stored_.get() + k * total;
   };
-  // Two passes per slice on the two-factor engine: k_slice_gradient (inverse rows, gradient, conj(screen),
-  // forward rows) and k_slice_cols<kSplitInv> (forward columns, split, inverse columns).
+  // Two passes per slice: slice_gradient (inverse rows, gradient, conj(screen), forward rows) and slice_cols with
+  // kSplitInv (forward columns, split, inverse columns).
   if (slice_covers(t_.n)) {
     const int groups = slice_groups(t_.n, nb);
     const auto split = [&](const float2* coef, int has_back, float* slice_grad) {
@@ -1174,7 +1175,7 @@ void BpmPlan::adjoint(const float* x, const float2* residual_or_null, int first,
       const float2* env = envelope(k);
       // Slice k's gradient groups are added by the next column pass, or here for the last slice.
       slice_gradient(t_.n, k > 0, w_.get(), env, x + k * plane_, t_.phase, inv, nb, gscale, gpart_.get(),
-                           k > 0 ? nullptr : grad, s);
+                     k > 0 ? nullptr : grad, s);
       if (k > 0) split(step_.get(), 1, grad + k * plane_);
     }
     return;
@@ -1210,7 +1211,7 @@ void BpmPlan::recompute(const float* x, int first, int nb, int k0, int k1, cudaS
   const float inv = 1.0f / static_cast<float>(plane_);
   const float2* ck = ckpt_.get() + (static_cast<std::size_t>(k0 / every_) * t_.count + first) * plane_;
   check(cudaMemcpyAsync(rs_.get(), ck, total * sizeof(float2), cudaMemcpyDeviceToDevice, s), "bpm restore");
-  // The forward sweep's two passes per slice (two-factor engine), so the envelopes are bitwise its own.
+  // The forward sweep's two passes per slice, so the envelopes are bitwise its own.
   if (slice_covers(t_.n)) {
     const auto screen = [&](int k) {  // rw_ holds C^-1(S) of slice k: envelope k, then its row FFT
       ColArgs w{};

@@ -721,8 +721,8 @@ void set_radix_tuning(bool on) { g_radix_tuning.store(on ? 1 : 0, std::memory_or
 namespace {
 
 // The engine where nothing is forced or tuned. 192 and 512 on the register engine hold 24 and 32 values a thread;
-// without the restore the two-factor engine is faster (192^3: y pass 12 us against 17; 512^3: 208 against 296,
-// from_data 265 against 317; with it 23 against 21 and 527 against 512).
+// without the restore the two-factor engine is faster (192^3: y pass 12 us against 17, from_data 10 against 12;
+// 512^3: 210 against 297 and 282 against 348; with it 23.5 against 20.6 and 526 against 517).
 int default_axis_engine(int n, AxisMode mode) {
   const bool restore = mode == AxisMode::restore_half || mode == AxisMode::restore_mask;
   if ((n == 192 || n == 512) && !restore && axis_two_covers(n)) return kTwoEngine;

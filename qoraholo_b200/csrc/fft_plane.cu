@@ -10,7 +10,7 @@
 //   1  y, radix R1: from global memory, position j + R2 q of column kx, to row k1 R2 + j
 //   2  y, radix R2: rows j2 R2 + (0 .. R2 - 1), after which row a R2 + b holds y = a + R1 b
 //   3  x, radix X1 (even), pairs of rows (i, i + n / 2) as one complex line of length n (their real rows are
-//      its real and imaginary parts, fft_two.cu): butterflies j and X2 - j together, since positions k and
+//      its real and imaginary parts): butterflies j and X2 - j together, since positions k and
 //      n - k come from the same two bins; value (k1, j) of the line goes to column j + X2 (k1 mod X1 / 2) of
 //      the first row (k1 < X1 / 2) or the second, which are bins that this pair of butterflies read
 //   4  x, radix X2 inverse, the constraint, radix X2 forward (factors exchanged), on one line's slots k1

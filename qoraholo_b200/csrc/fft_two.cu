@@ -6,10 +6,10 @@
 //
 // What bounds these passes is HBM (or L2) latency and bandwidth: a tile's loads are all issued at once
 // (16 to 32 per thread) and several CTAs share an SM, so one CTA's loads overlap another's transforms.
-// Measured on B200 against the staged passes: half spectrum of 384^3, y pass 96 us (4.7 TB/s) from 171, z pass
-// with the restore 205 us from 321; of 8 x 96^3, y 13 us from 32, z 22 us from 61; complex rows of 97 x 384^2
-// 53 us from 97. Lengths with a compile-time form on the register engine (fft_reg.cu) stay there: 256^3 y 27 us
-// against 30 here, z 53 against 63.
+// Measured on B200 against the staged passes: half spectrum of 384^3, y passes 89 and 95 us (5.1 and 4.8 TB/s) from
+// 171, z pass with the restore 196 us from 319; of 8 x 96^3, y 13 us from 33, z 19 us from 61; complex rows of
+// 97 x 384^2 52 us from 97. 64, 128 and 256, with a compile-time form on the register engine (fft_reg.cu), stay
+// there: 256^3 z with the restore 47 us against 54 here, y 26 against 25.
 #include "debug.cuh"
 #include "fft_rows.cuh"
 #include "fft_two.hpp"
@@ -334,7 +334,8 @@ __global__ void __launch_bounds__(256, min_blocks(Max))
 
 // The end of one FISTA-TV iteration and the start of the next on rows (fft3d.cu k_rows_tv_final_r2c: the
 // final primal, the momentum point, xprev, and the R2C of the momentum point), with the same operations;
-// the momentum point is formed with row-contiguous loads into shared memory, one warp per row at a time, 256^3: 93 us (470 MB, 5.0 TB/s) from 109; 150 x 180^2: 34 us from 48.
+// the momentum point is formed with row-contiguous loads into shared memory, one warp per row at a time. 256^3:
+// 92 us (470 MB, 5.1 TB/s) from 108; 150 x 180^2: 36 us from 48.
 template <int Max>
 __global__ void __launch_bounds__(256, min_blocks(Max))
     k_rows_tv_final_r2c_two(const float* __restrict__ b, const float* __restrict__ pz, const float* __restrict__ py,

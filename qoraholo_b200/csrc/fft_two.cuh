@@ -197,7 +197,10 @@ __device__ __forceinline__ void with_radix(int r, F&& f) {
   }
 }
 
-// The factors of a line length: r1 <= 16, r1 <= r2.
+// The factors of a line length. Kernels that give a line r2 threads (rows, axis passes, field columns, BPM slices)
+// need r1 <= r2, which `factors` (r1 up to 16, for with_first) and the field columns' own choice (r1 up to 32, for
+// with_radix) see to. The planes of fft_plane.cu stride their threads over the butterflies and need no order: their x
+// factors may have r1 > r2 (182 = 14 x 13).
 struct Factors {
   int r1 = 0, r2 = 0;
   __host__ __device__ int n() const { return r1 * r2; }

@@ -168,8 +168,9 @@ __global__ void __launch_bounds__(kThreads)
 // Passes 1 and 3 load their rows straight into the first DFT and leave through a natural-order copy in shared
 // memory, one warp per row, so that the window's split and the phase and log-amplitude run once per value on
 // coalesced rows. Pass 2 holds a column's spectrum only inside the crop window. Against the staged passes,
-// 200 x (192^2 -> 96^2): 20, 19 and 25 us from 40, 31 and 33; 49 x (400^2 -> 200^2): 27, 28 and 36 us from 36, 36
-// and 45; 97 x 1024^2 rows 196 us from 318 (the inverse rows of 384 217 from 203).
+// 200 x (192^2 -> 96^2): 20, 19 and 25 us from 39, 32 and 33; 49 x (400^2 -> 200^2): 27, 28 and 36 us from 35, 36
+// and 45; 97 x (1024^2 -> 384^2): 200, 117 and 218 from 317, 179 and 202. One image of 1024^2 -> 512^2: 9, 15 and 6 us
+// from 9, 12 and 8.
 
 using twofft::Factors;
 using twofft::RowTile;

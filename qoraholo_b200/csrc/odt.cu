@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(32 * kMapCols)
 // reconstruction; `measured` (optional) receives a second copy of the potential. One warp per lateral column,
 // as k_map_half with the column's own side only: every (column, view) target is computed once, where one
 // thread per 8 axial bins (k_map_full_bins, for nz above 1024) computes it nz / 8 times. Bounded by the ordered
-// sums; 49 views into 200^3: 37 us, 114 with a thread per 8 bins.
+// sums; 49 views into 200^3: 36 us, 116 with a thread per 8 bins.
 template <int kMapCols>
 __global__ void __launch_bounds__(32 * kMapCols)
     k_map_full(const float2* __restrict__ spectra, const float4* __restrict__ illum, int count, Grid g,

@@ -602,8 +602,8 @@ __global__ void __launch_bounds__(256)
 // and of dual step k are spread over all threads with the same point -> thread map in both phases,
 // so the step-k dual reads only z_k values that its own thread wrote in this iteration or that a
 // barrier separates from their writer: two barriers per plane. p_{k+1} and r_{k+1} of the thread's
-// own points stay in registers from dual step k to the z_{k+1} phase and dual step k + 1. The per-point operations are those of k_fgp in
-// the same order, so the iterates are bit-identical.
+// own points stay in registers from dual step k to the z_{k+1} phase and dual step k + 1. The per-point
+// operations are those of k_fgp in the same order, so the iterates are bit-identical.
 struct Fgp2Args {
   const float* pin[3];  // p_k (not read on the first step)
   float* pout[3];       // p_{k+2}
@@ -721,10 +721,11 @@ constexpr int fgp2_threads(int ty) { return ty >= 8 ? 512 : 256; }
 // CUBE > 0: compiled for a CUBE^3 volume (the sizes, the pitch and the block shape are constants, so
 // shared-memory and global addresses fold into immediate offsets); 0: any size, from the arguments.
 //
-// Window: tiles over x as well, for rows that do not fit one tile (two steps of 160 x 300 x 320 in 244 us, two
-// one-step passes 317), and taller tiles of shorter rows, up to what 512 threads and the shared memory hold:
+// Window: tiles over x as well, for rows that do not fit one tile (two steps of 160 x 300 x 320 in 209 us, two
+// one-step passes 319), and taller tiles of shorter rows, up to what 512 threads and the shared memory hold:
 // fewer halo rows and planes run ahead, against more work between the barriers of a plane (150 x 180^2, a
-// middle pair of steps: 85 us with 11 rows, 81 with 8, the last pair 62 and 72; the tuner picks). A window's
+// middle pair of steps: 74 us with 11 rows, 81 with 8, the last pair 65 and 72; 96^3 23.9 with 16, 22.8 with 8; the
+// tuner picks). A window's
 // results depend on the two columns beside it per side (one per step, and the shifted x differences), so it
 // computes four more columns on each side than it writes: what the outermost of them lack is not written,
 // and the box loads' x stays on 16 bytes.
@@ -865,7 +866,8 @@ __global__ void __launch_bounds__(fgp2_threads(TY), 1) k_fgp2(Fgp2Args A, const 
   const auto ld2 = [](const float* p) { return *reinterpret_cast<const float2*>(p); };
   const auto st2 = [](float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; };
 
-  const long long units = static_cast<long long>(CUBE > 0 ? (CUBE + TY - 1) / TY : Window ? A.ytiles * A.xtiles : A.ytiles) * nz;
+  const int tiles = CUBE > 0 ? (CUBE + TY - 1) / TY : Window ? A.ytiles * A.xtiles : A.ytiles;
+  const long long units = static_cast<long long>(tiles) * nz;
   const long long u_end = units * (blockIdx.x + 1) / gridDim.x;
   for (long long u = units * blockIdx.x / gridDim.x; u < u_end;) {
     const int tile = static_cast<int>(u / nz);
@@ -1166,7 +1168,9 @@ bool fgp2_fits(int nx, int ty) {
 struct Fgp2Window {
   int ty = 0, xtiles = 0, inner = 0, win = 0;
 };
-constexpr int kWindowRows[] = {16, 14, 12, 11, 10, 8};  // instantiated heights
+// Instantiated heights: each is the tallest of some widths (a middle pair against 8 rows, 16 at 128^3: 37 and 47 us, at
+// 78 x 112^2: 26 and 30; 11 at 150 x 180^2: 75 and 82; 10 at 192^3: 98 and 102).
+constexpr int kWindowRows[] = {16, 14, 12, 11, 10, 8};
 constexpr int kMaxWindows = 8;
 // The tallest tile with `xtiles` windows; ty = 0 when none fits.
 Fgp2Window fgp2_window(int nx, int xtiles) {
@@ -1327,7 +1331,7 @@ FgpShape fgp_shape(int nz, int ny, int nx, bool two_step) {
   const int form = g_fgp_form.load();
   const int fallback = fgp_rows_default<VEC>(nx);
   // Untuned, two steps per pass with the fewest tiles where the caller's buffers allow it (160 x 300 x 320, ten
-  // steps: 1.13 ms, in two windows of 11 rows, where the stored-r form took 1.56), else the stored-r form.
+  // steps: 1.14 ms, in two windows of 11 rows, where the stored-r form took 1.71), else the stored-r form.
   const Fgp2Window fewest = VEC == 4 && two_step ? fgp2_fewest_tiles(ny, nx) : Fgp2Window{};
   const int two = fewest.ty == 0                             ? fallback
                   : fewest.xtiles == 1 && fewest.ty == 8 ? 2 * kFgpVariantScale + 8
@@ -1344,7 +1348,8 @@ FgpShape fgp_shape(int nz, int ny, int nx, bool two_step) {
     if (smem > 200 * 1024) choice = (form - 1) * kFgpVariantScale + 1;
   }
   const int variant = choice / kFgpVariantScale, of = choice % kFgpVariantScale;
-  if (variant >= 2 && (VEC != 4 || !two_step || (variant == 2 ? !fgp2_fits(nx, of) : of < 1 || fgp2_window(nx, of).ty == 0))) {
+  const bool fits = variant == 2 ? fgp2_fits(nx, of) : of >= 1 && fgp2_window(nx, of).ty != 0;
+  if (variant >= 2 && (VEC != 4 || !two_step || !fits)) {
     choice = fallback;
   }
   return fgp_shape_rows<VEC>(nz, ny, nx, choice);

@@ -599,7 +599,7 @@ int unwrap_line_threads(int n) {
 // access has bank conflicts and no index needs a division. What bounds the passes is the latency of their
 // phases: 16 lines per tile up to a side of 320, 8 beyond, and in a stack kernels of the factors' class only.
 // 200 images of sides 96 .. 640 in steps of 8 (18 M pixels): the three passes take 0.9 ms, on the staged engine
-// 9.5 ms; 49 images of 200^2 26, 30 and 28 us from 33, 46 and 37; one of 120 x 160 27 us from 40.
+// 9.5 ms; 49 images of 200^2 27, 30 and 28 us from 33, 46 and 37; one of 120 x 160 26 us from 37.
 struct DctLine {
   int n = 0;  // side; 0: not on this engine
   int r1 = 0, r2 = 0;
@@ -954,7 +954,8 @@ bool pass1_two(const float* psi, float* d1, int count, int ny, int nx, const flo
   if (f.n == 0) return false;
   with_line_class(f, [&]<int Max>() {
     ensure_smem(k_div_dctx_two<Max>);
-    k_div_dctx_two<Max><<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(psi, d1, ny, f, twn, dtw);
+    const dim3 grid((ny + f.lines - 1) / f.lines, count);
+    k_div_dctx_two<Max><<<grid, kThreads, f.rows_smem(), s>>>(psi, d1, ny, f, twn, dtw);
   });
   check_launch("unwrap pass 1");
   return true;
@@ -965,8 +966,8 @@ bool pass2_two(const float* d1, float* phi, int count, int ny, int nx, const flo
   if (f.n == 0) return false;
   with_line_class(f, [&]<int Max>() {
     ensure_smem(k_dcty_solve_two<Max>);
-    k_dcty_solve_two<Max><<<dim3((nx + f.lines - 1) / f.lines, count), kThreads, f.cols_smem(), s>>>(d1, phi, nx, f, twn, dtw,
-                                                                                                cos_y, cos_x);
+    const dim3 grid((nx + f.lines - 1) / f.lines, count);
+    k_dcty_solve_two<Max><<<grid, kThreads, f.cols_smem(), s>>>(d1, phi, nx, f, twn, dtw, cos_y, cos_x);
   });
   check_launch("unwrap pass 2");
   return true;
@@ -977,16 +978,16 @@ bool pass3_two(float* phi, const float* psi, int count, int ny, int nx, const fl
   if (f.n == 0) return false;
   with_line_class(f, [&]<int Max>() {
     ensure_smem(k_idctx_two<Max>);
-    k_idctx_two<Max><<<dim3((ny + f.lines - 1) / f.lines, count), kThreads, f.rows_smem(), s>>>(phi, psi, ny, f, twn, dtw,
-                                                                                           partial);
+    const dim3 grid((ny + f.lines - 1) / f.lines, count);
+    k_idctx_two<Max><<<grid, kThreads, f.rows_smem(), s>>>(phi, psi, ny, f, twn, dtw, partial);
   });
   check_launch("unwrap pass 3");
   return true;
 }
 
 // Rows of a pass-1 / pass-3 tile and columns of a pass-2 tile for lines of length n: the register
-// engine's R = 256 / T where it runs, the two-factor tiles' lines, else the staged tiles'. Every path (planned, batched, without
-// allocation) tiles alike, so that the congruence partial sums, and with them the results, agree.
+// engine's R = 256 / T where it runs, the two-factor tiles' lines, else the staged tiles'. Every path (planned,
+// batched, without allocation) tiles alike, so that the congruence partial sums, and with them the results, agree.
 int rows_per_cta(int len, std::size_t extra_per_row);
 
 int unwrap_tile_rows(int nx) {
@@ -1353,7 +1354,8 @@ __global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.nx, QHK_R1)
     } else if constexpr (Kind == kTwo) {
-      div_dctx_tile_two<twofft::kAny>(psi + im.offset, d1 + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, sm);
+      div_dctx_tile_two<twofft::kAny>(psi + im.offset, d1 + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x,
+                                      w.y * im.line_x.lines, sm);
     } else {
       QHK_ROWS_SWITCH(im.rows, QHK_P1)
     }
@@ -1380,8 +1382,8 @@ __global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.ny, QHK_R2)
     } else if constexpr (Kind == kTwo) {
-      dcty_solve_tile_two<twofft::kAny>(d1 + im.offset, phi + im.offset, im.nx, im.line_y, im.Ly.tw, im.dtw_y, im.cos_y, im.cos_x,
-                          w.y * im.line_y.lines, sm);
+      dcty_solve_tile_two<twofft::kAny>(d1 + im.offset, phi + im.offset, im.nx, im.line_y, im.Ly.tw, im.dtw_y,
+                                        im.cos_y, im.cos_x, w.y * im.line_y.lines, sm);
     } else {
       QHK_ROWS_SWITCH(im.cols, QHK_P2)
     }
@@ -1409,8 +1411,8 @@ __global__ void __launch_bounds__(kThreads, Kind == kStaged ? 1 : 2)
     if constexpr (Kind == kReg) {
       QHK_REG_SWITCH(im.nx, QHK_R3)
     } else if constexpr (Kind == kTwo) {
-      idctx_tile_two<twofft::kAny>(phi + im.offset, psi + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x, w.y * im.line_x.lines, pair,
-                     sm, red);
+      idctx_tile_two<twofft::kAny>(phi + im.offset, psi + im.offset, im.ny, im.line_x, im.Lx.tw, im.dtw_x,
+                                   w.y * im.line_x.lines, pair, sm, red);
     } else {
       QHK_ROWS_SWITCH(im.rows, QHK_P3)
     }
@@ -1589,7 +1591,9 @@ UnwrapBatchPlan::UnwrapBatchPlan(const int* ny, const int* nx, int count) {
     for (int t = 0; t < (b.nx + b.cols - 1) / b.cols; ++t) items[3 * b.kind_y + 1].push_back(make_int2(i, t));
     items[kConstsPass].push_back(make_int2(i, 0));
     const std::size_t pixels = static_cast<std::size_t>(b.ny) * b.nx;
-    for (std::size_t t = 0; t * kAssembleChunk < pixels; ++t) items[kConstsPass + 1].push_back(make_int2(i, static_cast<int>(t)));
+    for (std::size_t t = 0; t * kAssembleChunk < pixels; ++t) {
+      items[kConstsPass + 1].push_back(make_int2(i, static_cast<int>(t)));
+    }
   }
   for (const int kind : {kStaged, kReg, kTwo}) items[3 * kind + 2] = items[3 * kind];
   std::vector<int2> all;

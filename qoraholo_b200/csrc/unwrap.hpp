@@ -35,11 +35,11 @@ class UnwrapPlan {
 
 // Least-squares unwrap of an uneven batch: `count` images, image i of its own (even) size ny[i] x
 // nx[i], packed one after another in the input and output buffers (image i starts at offset(i) =
-// the pixel count of images 0 .. i-1). Each of the five passes is ONE launch for the whole batch:
-// persistent CTAs (as many as are resident at once) take (image, tile) items off a device queue,
-// largest images first, and run the tile code of the stacked plan above for that image's size, so
-// every image's result is bitwise the one UnwrapPlan gives for it. unwrap_graph replays the five
-// launches as one captured CUDA graph.
+// the pixel count of images 0 .. i-1). Passes 4 and 5 are one launch each for the whole batch, passes
+// 1 to 3 one per FFT engine that some image's lines take (at most three): persistent CTAs (as many as
+// are resident at once) take (image, tile) items off a device queue, largest images first, and run the
+// tile code of the stacked plan above for that image's size, so every image's result is bitwise the one
+// UnwrapPlan gives for it. unwrap_graph replays the launches as one captured CUDA graph.
 class UnwrapBatchPlan {
  public:
   UnwrapBatchPlan(const int* ny, const int* nx, int count);

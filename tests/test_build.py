@@ -23,7 +23,10 @@ def build():
 def test_other_flags_make_an_object_stale(build, tmp_path):
     src, obj = tmp_path / "a.cpp", tmp_path / "a.o"
     src.write_text("int a() { return 1; }\n")
-    command = lambda *flags: ["g++", *flags, "-MD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)]  # noqa: E731
+
+    def command(*flags):
+        return ["g++", *flags, "-MD", "-MF", str(obj.with_suffix(".d")), "-c", str(src), "-o", str(obj)]
+
     assert build._stale(obj, src, command("-O1"))
     build._compile(command("-O1"))
     assert not build._stale(obj, src, command("-O1"))

@@ -64,7 +64,8 @@ def _gp_against_the_oracle(torch, n, nz, amplitude):
 
     il = O.circular_scan(3, 0.9, G)
     rng = np.random.default_rng(n)
-    fields = (rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n))).astype(np.complex64) * np.float32(amplitude)
+    fields = (rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n))).astype(np.complex64)
+    fields *= np.float32(amplitude)
     want, _ = O.reconstruct(fields, il, G, nz=nz, iterations=2)
     plan = capi.OdtPlan(n, 3, il, G, nz=nz, iterations=2)
     d, out = torch.from_numpy(fields).cuda(), torch.empty(plan.shape, dtype=torch.float32, device="cuda")
